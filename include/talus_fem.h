@@ -202,8 +202,10 @@ int32_t tl_system_tune_shape(tl_system* system, uint32_t knob, uint32_t value);
  * the 3x3 node blocks once per solve and iterates on that matrix (about 40
  * bytes per nonzero block in FP32, 76 in FP64);
  * TL_SOLVER_ELEMENTWISE always iterates element by element;
- * TL_SOLVER_AUTO (default) is ASSEMBLED for batched systems and for single
- * bodies of at least 32,768 tets, ELEMENTWISE for smaller single bodies.
+ * TL_SOLVER_AUTO (default) is ASSEMBLED for batched systems, for single
+ * bodies of up to 5,120 nodes (which then solve inside one thread-block
+ * cluster, kPcgCluster, where their rows fit its shared memory) and for single
+ * bodies of at least 32,768 tets, ELEMENTWISE for the single bodies between.
  * Both forms apply the same operator; they differ in rounding.  On the
  * assembled matrix a batch (or a body too large for the single-body grid)
  * iterates in one of two orders with the same iterates in exact arithmetic:

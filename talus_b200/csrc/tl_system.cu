@@ -9,6 +9,7 @@
 #include "tl_adjoint.cuh"
 #include "tl_floating.cuh"
 #include "tl_sell.cuh"
+#include "tl_cluster.cuh"
 #include "tl_sell_build.h"
 #include "tl_factor.cuh"
 #include "tl_factor_host.h"
@@ -236,6 +237,7 @@ struct tl_ctx {
   cudaStream_t stream = nullptr;
   int sms = 0;
   std::string last_error;
+  int clusterFits[2][2] = {{-1, -1}, {-1, -1}};  // whether the device runs kPcgCluster, [FP64][K - 1]; -1: not asked yet
 };
 
 struct RolloutBase {
@@ -939,6 +941,93 @@ struct System final : SystemBase {
     }
     TL_CUDA(cudaStreamSynchronize(st));
     sellReady = sellPerSm > 0 || batchSellPerSm > 0;
+    buildCluster(h);
+  }
+  // The body's rows over the blocks of one cluster (kPcgCluster).
+  struct ClusterPlan {
+    const void* kernel = nullptr;  // null: none
+    size_t smem = 0;
+    ClusterDev dev{};
+  };
+  ClusterPlan cluster;
+  DevBuf<unsigned char> clArrays;  // the partition (ClusterHost), packed
+  cudaLaunchConfig_t clusterConfig(cudaLaunchAttribute* at) const {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(CLUSTER_MAX);
+    cfg.blockDim = dim3(CLUSTER_T);
+    cfg.dynamicSmemBytes = cluster.smem;
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = CLUSTER_MAX;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+  }
+  // One body whose rows fit the blocks of a cluster of 16: up to 10 slices a block, 5,120 rows.  At 4,624 rows an
+  // iteration takes 7.0 us where the whole-GPU kernels take 7.7 (FP32-mixed) and 9.0 us (FP64), at 3,840 4.9
+  // against 7.7 and 8.9, at 1,331 2.3 against 7.5 and 8.4.  More rows find no worker for every slice and fewer of
+  // their blocks on the SM.  16 blocks beat 8 and 4 from 250 rows up and equal them below.
+  void buildCluster(const SellHost& h) {
+    cluster = ClusterPlan{};
+    if (B != 1) return;
+    const uint32_t perBlock = std::max(1u, (h.slices + CLUSTER_MAX - 1) / CLUSTER_MAX);
+    const uint32_t rows = perBlock <= CLUSTER_OWNERS ? 1u : 2u;  // an owner's slices
+    const uint32_t owners = (perBlock + rows - 1) / rows;
+    if (owners > CLUSTER_OWNERS || perBlock > CLUSTER_W - owners) return;  // a worker for every slice
+    ClusterHost c;
+    if (!buildClusterHost(h, CLUSTER_MAX, c)) return;
+    ClusterDev& d = cluster.dev;
+    d.slices = perBlock;
+    d.owners = owners;
+    d.parts = std::min(CLUSTER_PARTS, (CLUSTER_W - owners) / perBlock);
+    d.entries = c.maxEntries;
+    d.positions = c.maxPositions;
+    int limit = 0;
+    TL_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    const uint32_t perWorker = (h.widest + d.parts - 1) / d.parts;  // column slots of a worker's slice
+    d.cached = perWorker > CLUSTER_REG ? perWorker - CLUSTER_REG : 0u;
+    while (d.cached > 0 && clusterLayout(d, d.cached).total > size_t(limit)) --d.cached;
+    d.far = perWorker > CLUSTER_REG + d.cached ? 1u : 0u;
+    cluster.smem = clusterLayout(d, d.cached).total;
+    if (cluster.smem > size_t(limit)) return;
+    const void* const fn = rows == 1 ? (const void*)kPcgCluster<S, 1> : (const void*)kPcgCluster<S, 2>;
+    int& fitsDevice = ctx->clusterFits[sizeof(S) == 8 ? 1 : 0][rows - 1];
+    if (fitsDevice < 0) {  // once per context: the attributes are the kernel's, so they cover every system
+      TL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+      TL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      cudaLaunchAttribute at[1];
+      cudaLaunchConfig_t cfg = clusterConfig(at);
+      cfg.dynamicSmemBytes = size_t(limit);
+      int active = 0;
+      if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess) cudaGetLastError();
+      fitsDevice = active > 0 ? 1 : 0;
+    }
+    if (!fitsDevice) return;
+    // one buffer for the partition's arrays, each from a 16-byte boundary
+    std::vector<unsigned char> packed;
+    const auto put = [&](const auto& src) {
+      const size_t at = packed.size(), bytes = src.size() * sizeof(src[0]);
+      packed.resize(at + (bytes + 15) / 16 * 16 + 16);
+      std::memcpy(packed.data() + at, src.data(), bytes);
+      return at;
+    };
+    const size_t foreign = put(c.foreign), local = put(c.local), push = put(c.push), overStart = put(c.overStart),
+                 over = put(c.over);
+    clArrays.alloc(packed.size());
+    clArrays.upload(packed.data(), packed.size(), st);
+    TL_CUDA(cudaStreamSynchronize(st));
+    static_assert(CLUSTER_INLINE == 4, "a row's inline destinations are one uint4");
+    d.foreign = reinterpret_cast<const uint32_t*>(clArrays.ptr + foreign);
+    d.local = reinterpret_cast<const uint16_t*>(clArrays.ptr + local);
+    d.push = reinterpret_cast<const uint4*>(clArrays.ptr + push);
+    d.over_start = reinterpret_cast<const uint32_t*>(clArrays.ptr + overStart);
+    d.over = reinterpret_cast<const uint32_t*>(clArrays.ptr + over);
+    cluster.kernel = fn;
+  }
+  // Whether this system's solves run in a cluster.
+  bool clusterForm() const {
+    return sellReady && cluster.kernel && (solverForm == TL_SOLVER_AUTO || solverForm == TL_SOLVER_ASSEMBLED);
   }
   size_t sellColBytes() const { return size_t(sellColCache) * TILE * sizeof(uint32_t); }
   void assembleSell(const Sys<S>& s, const SellDev<S>& g, unsigned blocks, int idx, bool damp, bool tangent,
@@ -1410,16 +1499,34 @@ struct System final : SystemBase {
       pcgFactor(law, X, pass, x0zero, tangent);
       return;
     }
-    kPcgPrepare<S><<<1, TILE, 0, st>>>(view(), pass);
-    check();
+    if (!clusterForm()) {  // the grid barrier's words
+      kPcgPrepare<S><<<1, TILE, 0, st>>>(view(), pass);
+      check();
+    }
     Sys<S> s = view();
     uint32_t ps = pass, xz = x0zero ? 1u : 0u, tg = tangent ? 1u : 0u;
     const int idx = law == TL_LAW_SNH ? 1 : 0;
     const size_t dyn = idx ? (tangent ? pipeBytes<S, 1, true>() : pipeBytes<S, 1, false>())
                            : (tangent ? pipeBytes<S, 0, true>() : pipeBytes<S, 0, false>());
     const bool damp = hasDamping && idx == 0;
-    const int sellG = sellGrid();
-    if (sellG > 0) {  // single body: assembled block matrix, pipelined PCG
+    const bool inCluster = clusterForm();
+    const int sellG = inCluster ? 0 : sellGrid();
+    if (inCluster) {  // single body that fits a cluster
+      SellDev<S> g = sellView();
+      const unsigned blocks = (sellUpperCount + TILE - 1) / TILE;
+      if (profiling) mark(1, true);
+      assembleSell(s, g, blocks, idx, damp, tangent, ps);
+      check();
+      if (profiling) {
+        mark(1, false);
+        mark(2, true);
+      }
+      ClusterDev c = cluster.dev;
+      void* args[] = {&s, &g, &c, &X, &xz, &tg};
+      cudaLaunchAttribute at[1];
+      const cudaLaunchConfig_t cfg = clusterConfig(at);
+      TL_CUDA(cudaLaunchKernelExC(&cfg, cluster.kernel, args));
+    } else if (sellG > 0) {  // single body: assembled block matrix, pipelined PCG
       SellDev<S> g = sellView();
       const unsigned blocks = (sellUpperCount + TILE - 1) / TILE;
       if (profiling) mark(1, true);  // the operator assembly counts as assembly time
