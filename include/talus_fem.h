@@ -190,9 +190,9 @@ int32_t tl_system_tune(tl_system* system, uint32_t pcg_blocks_per_sm, uint32_t g
  * (chosen by talus_b200/autotune.py); results are bitwise the same for every
  * shape. TL_SHAPE_ROW_GROUP: column slots of a matrix row whose inputs and
  * blocks are requested per round trip, 2 or 4 (0 = the default: 4 in FP32
- * and 2 in FP64 for a single body, 2 for batches). TL_SHAPE_BATCH_BLOCKS:
- * resident 256-thread blocks per SM the batched kernels are compiled for,
- * 3 or 4 (0 = 4). Other values return TL_ERR_ARG. */
+ * and 2 in FP64, 2 in the lockstep batched orders). TL_SHAPE_BATCH_BLOCKS:
+ * resident 256-thread blocks per SM the lockstep batched kernels are compiled
+ * for, 3 or 4 (0 = 4). Other values return TL_ERR_ARG. */
 #define TL_SHAPE_ROW_GROUP 0u
 #define TL_SHAPE_BATCH_BLOCKS 1u
 int32_t tl_system_tune_shape(tl_system* system, uint32_t knob, uint32_t value);
@@ -207,14 +207,15 @@ int32_t tl_system_tune_shape(tl_system* system, uint32_t knob, uint32_t value);
  * cluster, kPcgCluster, where their rows fit its shared memory) and for single
  * bodies of at least 32,768 tets, ELEMENTWISE for the single bodies between.
  * Both forms apply the same operator; they differ in rounding.  On the
- * assembled matrix a batch (or a body too large for the single-body grid)
- * iterates in one of two orders with the same iterates in exact arithmetic:
- * TL_SOLVER_ASSEMBLED_TWO_PHASE, the textbook order with two grid barriers
- * per iteration, or TL_SOLVER_ASSEMBLED_PIPELINED, the pipelined order with
- * one barrier per iteration and its recurrences kept in FP64 (eight vectors
- * per node, in both precisions). ASSEMBLED and AUTO take the pipelined order
- * in FP64 and the two-phase order in FP32-mixed, the faster of each on the
- * 512-body batch. */
+ * assembled matrix ASSEMBLED and AUTO iterate each body of a batch with its
+ * own group of blocks, in the pipelined order with one barrier per iteration
+ * and its recurrences in FP64 registers (kPcgSell).  Two other orders, with
+ * the same iterates in exact arithmetic, step every body of the system in
+ * lockstep: TL_SOLVER_ASSEMBLED_TWO_PHASE, the textbook order with two grid
+ * barriers per iteration, and TL_SOLVER_ASSEMBLED_PIPELINED, the pipelined
+ * order with its recurrences in memory (eight FP64 vectors per node).  A
+ * system with a body of more nodes than the resident grid has threads takes
+ * the pipelined one in FP64 and the two-phase one in FP32-mixed. */
 #define TL_SOLVER_AUTO 0u
 #define TL_SOLVER_ASSEMBLED 1u
 #define TL_SOLVER_ELEMENTWISE 2u

@@ -139,7 +139,7 @@ struct GridSyncDev {
   int error;
   int active;      // bodies still iterating in the current PCG solve
   int active_odd;  // its copy for odd phases of the one-barrier batched PCG (kPcgBatchSellPipe)
-  int pad;
+  unsigned int ticket;  // bodies handed out to the clusters of kPcgCluster beyond their first
 };
 
 // Per-element matvec operator, one record per element: the gradients
@@ -1899,9 +1899,8 @@ __device__ __forceinline__ bool countBarrier(GridSyncDev* sync, unsigned int& k)
 // warp and the warps in order, so a grid barrier is followed by one L2 round
 // trip instead of one per block stride.
 template <int N>
-__device__ __forceinline__ void sumBlocksAll(const double* part, double (&out)[N]) {
+__device__ __forceinline__ void sumBlocksAll(const double* part, double (&out)[N], unsigned G = gridDim.x) {
   __shared__ double red[N][TILE / 32];
-  const unsigned G = gridDim.x;
   double v[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) v[k] = 0.0;
@@ -1931,17 +1930,16 @@ __device__ __forceinline__ void sumBlocksAll(const double* part, double (&out)[N
 // committed as one group; the caller waits for it (cp.async.wait_group 0),
 // then a block barrier, before sumStagedBlocks reads them.  part is 16-byte
 // aligned and holds at least fields G + 1 values.
-__device__ __forceinline__ void requestBlockPartials(const double* part, double* stage, unsigned fields) {
-  const unsigned pieces = (fields * gridDim.x + 1u) / 2u;
+__device__ __forceinline__ void requestBlockPartials(const double* part, double* stage, unsigned fields, unsigned G) {
+  const unsigned pieces = (fields * G + 1u) / 2u;
   for (unsigned i = threadIdx.x; i < pieces; i += TILE) cpAsync<16>(stage + 2 * i, part + 2 * i);
   cpAsyncCommit();
 }
 // sumBlocksAll on partials staged by requestBlockPartials: the same order of
 // additions, so the same sums.
 template <int N>
-__device__ __forceinline__ void sumStagedBlocks(const double* stage, double (&out)[N]) {
+__device__ __forceinline__ void sumStagedBlocks(const double* stage, double (&out)[N], unsigned G) {
   __shared__ double red[N][TILE / 32];
-  const unsigned G = gridDim.x;
   double v[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) v[k] = 0.0;
@@ -2733,6 +2731,7 @@ __global__ void kPcgPrepare(Sys<S> s, uint32_t pass) {
     s.sync->arrive = 0u;
     s.sync->active = count;
     s.sync->active_odd = count;
+    s.sync->ticket = 0u;
   }
 }
 

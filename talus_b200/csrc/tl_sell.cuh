@@ -14,14 +14,14 @@
 //                  land there (FP64 accumulation, stored in S), written with
 //                  its transpose below the diagonal; the diagonal blocks are
 //                  written by kNodeAssemble;
-//   kPcgBatchSell  the batched PCG on this matrix, for batches and for
-//                  single bodies with more rows than kPcgSell's grid has
-//                  threads, in the textbook order (two grid barriers per
-//                  iteration): the order of FP32-mixed systems;
+//   kPcgBatchSell  the batched PCG on this matrix in the textbook order (two
+//                  grid barriers per iteration), for systems with a body of
+//                  more rows than kPcgSell's grid has threads (FP32-mixed),
+//                  or by choice;
 //   kPcgBatchSellPipe  the same solve in kPcgSell's pipelined arrangement
 //                  with per-body scalars, one grid barrier per iteration and
-//                  its recurrences in FP64: the order of FP64 systems;
-//   kPcgSell       (one body) persistent cooperative PCG in the pipelined arrangement
+//                  its recurrences in FP64 (for such systems in FP64);
+//   kPcgSell       persistent cooperative PCG in the pipelined arrangement
 //                  of Ghysels and Vanroose ("Hiding global synchronization
 //                  latency in the preconditioned conjugate gradient
 //                  algorithm", 2014), which overlaps the one reduction of an
@@ -29,6 +29,8 @@
 //                  barrier.  Each thread owns one node row and keeps its
 //                  vectors in FP64 registers; only the matvec input is
 //                  published (rounded to S, and used rounded on both sides).
+//                  In a batch each body is iterated by just enough blocks,
+//                  which take bodies from a queue.
 //
 // Layout: sliced ELL with 32 rows per slice (one warp).  Slice s holds its
 // rows' blocks in width_s columns; block position p = slice_start[s] +
@@ -56,6 +58,7 @@ template <class S> struct SellDev {
   const uint32_t* col;           // [positions] column node
   uint32_t upper_count;          // block positions with row < column
   uint32_t col_cache;            // column slots per thread kept in shared memory by kPcgSell
+  uint32_t kept;                 // column slots whose blocks kPcgSell keeps in shared memory too
   // [upper_count] per block above the diagonal: (position, its transpose's position, first
   // contributor, contributor count | row free << 8 | column free << 9 | body << 10)
   const uint4* urec;
@@ -232,17 +235,88 @@ template <class S> struct Ld4cg {
   __device__ __forceinline__ Vec4<S> operator()(uint32_t c) const { return ld4cg(&v[c]); }
 };
 template <class S> __device__ __forceinline__ Ld4cg<S> ld4cgOf(const Vec4<S>* v) { return Ld4cg<S>{v}; }
-// kPcgSell's row: columns from its shared-memory cache, no prefetch, U slots per round trip.
+// kPcgSell's row: columns from its shared-memory cache, no prefetch, U slots
+// per round trip, the blocks of its first `kept` slots (a multiple of U) from
+// shared memory.
 template <class S, uint32_t U>
 __device__ __forceinline__ V3<double> sellRow(const SellDev<S>& g, uint32_t slice, uint32_t lane,
-                                              const Vec4<S>* in, const uint32_t* cols) {
-  return sellRowOf<S, Ld4cg<S>, U, false>(g, slice, lane, ld4cgOf(in), cols);
+                                              const Vec4<S>* in, const uint32_t* cols, const S* near, uint32_t kept) {
+  V3<double> acc = {0, 0, 0};
+  const uint32_t p1 = __ldg(&g.slice_start[slice + 1]);
+  uint32_t p = __ldg(&g.slice_start[slice]) + lane, k = 0;
+  for (; k < kept && p + (U - 1) * SELL_ROWS < p1; p += U * SELL_ROWS, k += U) {
+    Vec4<S> xin[U];
+#pragma unroll
+    for (uint32_t i = 0; i < U; ++i) xin[i] = ld4cg(&in[sellCol(cols, g.col_cache, k + i, g.col, p + i * SELL_ROWS)]);
+#pragma unroll
+    for (uint32_t i = 0; i < U; ++i) {
+      const S* const v = near + size_t(k + i) * 9 * SELL_ROWS;
+      const V3<double> x = cvt<double>(xyz(xin[i]));
+      acc.x = fma(double(v[0]), x.x, fma(double(v[32]), x.y, fma(double(v[64]), x.z, acc.x)));
+      acc.y = fma(double(v[96]), x.x, fma(double(v[128]), x.y, fma(double(v[160]), x.z, acc.y)));
+      acc.z = fma(double(v[192]), x.x, fma(double(v[224]), x.y, fma(double(v[256]), x.z, acc.z)));
+    }
+  }
+  for (; p + (U - 1) * SELL_ROWS < p1; p += U * SELL_ROWS, k += U) {
+    uint32_t c[U];
+#pragma unroll
+    for (uint32_t i = 0; i < U; ++i) c[i] = sellCol(cols, g.col_cache, k + i, g.col, p + i * SELL_ROWS);
+    Vec4<S> xin[U];
+#pragma unroll
+    for (uint32_t i = 0; i < U; ++i) xin[i] = ld4cg(&in[c[i]]);
+#pragma unroll
+    for (uint32_t i = 0; i < U; ++i) sellSlot(g, p + i * SELL_ROWS, lane, xin[i], acc);
+  }
+  for (; p < p1; p += SELL_ROWS, ++k) sellSlot(g, p, lane, ld4cg(&in[sellCol(cols, g.col_cache, k, g.col, p)]), acc);
+  return acc;
 }
 // Column slots per round trip of the assembled matvec rows (a launch shape
 // tl_system_tune_shape may change): kPcgSell's default, then the batched kernels'.
 template <class S> __host__ __device__ constexpr uint32_t sellRowGroup() { return sizeof(S) == 4 ? 4u : 2u; }
 constexpr uint32_t BATCH_ROW_GROUP = 2u;
 constexpr int BATCH_BLOCKS = 4;  // resident blocks per SM the batched kernels are compiled for by default
+
+// The bodies' rows over the blocks of kPcgSell: each body is `parts` items,
+// consecutive in the queue, and the blocks that take them iterate together.
+struct GangDev {
+  uint32_t items;
+  const uint4* item;  // [items] body, part, the body's first item, its parts
+  const uint2* body;  // [bodies] first slice, slices
+};
+
+// Counting barrier of a body's blocks: as countBarrier, with the body's own
+// arrival counter (zeroed before the launch).
+__device__ __forceinline__ bool gangBarrier(unsigned int* arrive, uint32_t parts, GridSyncDev* sync, unsigned int& k) {
+  __shared__ int ok;
+  ++k;
+  __syncthreads();
+  if (parts == 1u) return true;
+  if (threadIdx.x == 0) {
+    int good = 1;
+    const unsigned int goal = parts * k;
+    redAddRelease(arrive, 1u);
+    if (ldAcquire(arrive) < goal) {
+      const unsigned long long t0 = globalTimer();
+      unsigned int polls = 0;
+      while (ldAcquire(arrive) < goal) {
+        if ((++polls & 255u) == 0u) {
+          if (*(volatile int*)&sync->error != 0) {
+            good = 0;
+            break;
+          }
+          if (globalTimer() - t0 > TL_BARRIER_LIMIT_NS) {
+            atomicExch(&sync->error, 5);  // TL_ERR_TIMEOUT
+            good = 0;
+            break;
+          }
+        }
+      }
+    }
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
 
 template <class S> __device__ __forceinline__ V3<double> roundTo(V3<double> v) {
   return cvt<double>(cvt<S>(v));
@@ -262,182 +336,221 @@ template <class S> __device__ __forceinline__ V3<double> roundTo(V3<double> v) {
 // update), the breakdown test (p.A p > 0 and r.u > 0) and the iteration
 // count are the reference's, and a solve that reaches the cap applies its
 // last update without a matvec.  Block partials are added in block order, so
-// every block takes the same decisions.  The slices of block b are
-// [b slices / G, (b + 1) slices / G), at most 8, one per warp.
-template <class S, uint32_t U = sellRowGroup<S>()>
-__global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Vec4<S>* X, uint32_t x0zero, uint32_t tangent) {
-  const uint32_t G = gridDim.x, lane = threadIdx.x & 31u;
-  const uint32_t s0 = uint32_t(uint64_t(blockIdx.x) * g.slices / G);
-  const uint32_t s1 = uint32_t(uint64_t(blockIdx.x + 1) * g.slices / G);
-  const uint32_t slice = s0 + (threadIdx.x >> 5);
-  const bool mine = slice < s1;
-  const uint32_t row = slice * SELL_ROWS + lane;
-  const bool live = mine && row < g.rows;
-  const bool freeRow = live && !s.anch[row];
-  const BodyStepDev st = s.step[0];
-  extern __shared__ uint32_t tlCols[];  // [col_cache][TILE] the first columns of each thread's row
+// every block takes the same decisions.  The slices of a body's part q of G are
+// [q slices / G, (q + 1) slices / G), at most 8, one per warp.
+//
+// One body (GANG false): the whole grid is its G parts.  A batch: every body
+// is split into items of up to 256 rows, consecutive in one queue, and a block
+// takes the next item, works it to the end of the solve with the blocks that
+// hold the body's other items, and takes the next.  Items are handed out in
+// order to resident blocks, so the parts of the oldest unfinished body are
+// always all held or free to be taken, and no wait is for a block that does not
+// run.  Bodies that converged cost nothing more, the vectors stay in registers,
+// and only the bodies in work (75,776 rows, 41 MB of FP32 matrix) take L2: 96
+// uneven bodies solved to 1e-6 take 15 ms where the lockstep kernel's 51 stream
+// every body from HBM, in FP64 at the default settings 7.6 against 18.
+//
+// The blocks of a row's first `kept` column slots stay in shared memory for the
+// solve: 8 of 15 in FP32, 4 in FP64, as far as two blocks per SM leave room.
+// An SM's matvec reads 400 KB (FP32) to 830 KB through a 64-byte-a-clock port,
+// so this takes 5% off a single body's iteration (9.0 -> 8.7 us at 393,216
+// tets) and 32% off an FP64 batch, whose bodies in work (82 MB) also stop
+// falling out of L2; 8% off an FP32-mixed one.
+template <class S, bool GANG, uint32_t U = sellRowGroup<S>()>
+__global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, GangDev gang, Vec4<S>* X, uint32_t pass, uint32_t x0zero, uint32_t tangent) {
+  const uint32_t lane = threadIdx.x & 31u;
+  // [col_cache][TILE] the first columns of each thread's row, then [TILE / 32][g.kept][9][32] its warp's first blocks
+  extern __shared__ __align__(16) uint32_t tlCols[];
+  const uint32_t kept = g.kept;
+  S* const near = reinterpret_cast<S*>(tlCols + g.col_cache * TILE) + size_t(threadIdx.x >> 5) * kept * 9 * SELL_ROWS + lane;
   // the block partials of each iteration's reduction, fetched while the matvec's inputs are
   // (grids of up to SELL_PART_STAGE_BLOCKS blocks; larger ones read them from L2 after it)
   constexpr unsigned SELL_PART_STAGE_BLOCKS = 320;
   __shared__ __align__(16) double partStage[3 * SELL_PART_STAGE_BLOCKS + 2];
-  const bool stagedSums = G <= SELL_PART_STAGE_BLOCKS;
-  if (mine) {
-    const uint32_t p0 = __ldg(&g.slice_start[slice]) + lane, p1 = __ldg(&g.slice_start[slice + 1]);
-    for (uint32_t k = 0, p = p0; k < g.col_cache && p < p1; ++k, p += SELL_ROWS)
-      tlCols[k * TILE + threadIdx.x] = __ldg(&g.col[p]);
-  }
-  __syncthreads();
-  // Block partials alternate between two halves of blk_part by reduction
-  // parity: with one barrier per iteration, a block may write the next
-  // reduction's partials while another still sums the previous one.
-  double* const halves[2] = {s.blk_part, s.blk_part + 4 * size_t(G)};
-  uint32_t reductions = 0;
-  unsigned int bar = 0;
-  Sym<S> Ps = {1, 1, 1, 0, 0, 0};  // the row's preconditioner block, widened where used
-  const auto precondition = [&](V3<double> v) {
-    const Sym<double> P = {double(Ps.xx), double(Ps.yy), double(Ps.zz), double(Ps.xy), double(Ps.xz), double(Ps.yz)};
-    return roundTo<S>(symMul(P, v));
-  };
-  V3<double> x = {0, 0, 0}, r = {0, 0, 0}, rhs = {0, 0, 0};
-  if (live) {
-    const Vec4<S> q0 = s.pre0[row], q1 = s.pre1[row];
-    Ps = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
-    rhs = cvt<double>(xyz(s.right[row]));
-    if (!x0zero) x = cvt<double>(xyz(X[row]));
-  }
-  uint32_t applications = 0;
-  // ---- r = right - A x (anchored rows 0), u = P r, published to vec[1]
-  if (!x0zero) {
-    const V3<double> ax = mine ? sellRow<S, U>(g, slice, lane, X, tlCols) : V3<double>{0, 0, 0};
-    if (freeRow) r = rhs - ax;
+  __shared__ uint32_t queued[2];  // two, as a block may pass over an item without a barrier
+  for (uint32_t turn = 0;; ++turn) {
+    uint32_t item = blockIdx.x;  // the block's first item, then the queue's
+    if (GANG && turn) {
+      if (gridDim.x >= gang.items) break;
+      if (threadIdx.x == 0) queued[turn & 1u] = gridDim.x + atomicAdd(&s.sync->ticket, 1u);
+      __syncthreads();
+      item = queued[turn & 1u];
+    }
+    if (GANG ? item >= gang.items : turn != 0u) break;
+    // body, part, the body's first item, its parts
+    const uint4 it = GANG ? __ldg(&gang.item[item]) : make_uint4(0u, blockIdx.x, 0u, gridDim.x);
+    const uint32_t b = it.x, part = it.y, G = it.w;
+    if (GANG && !bodyActive(s, b, pass)) continue;
+    const uint2 range = GANG ? __ldg(&gang.body[b]) : make_uint2(0u, g.slices);
+    const uint32_t slice = range.x + uint32_t(uint64_t(part) * range.y / G) + (threadIdx.x >> 5);
+    const bool mine = slice < range.x + uint32_t(uint64_t(part + 1u) * range.y / G);
+    const uint32_t row = slice * SELL_ROWS + lane;
+    const bool live = mine && row < (GANG ? s.body[b].node_end : g.rows);
+    const bool freeRow = live && !s.anch[row];
+    const BodyStepDev st = s.step[b];
+    const bool stagedSums = G <= SELL_PART_STAGE_BLOCKS;
+    if (mine) {
+      const uint32_t p0 = __ldg(&g.slice_start[slice]) + lane, p1 = __ldg(&g.slice_start[slice + 1]);
+      for (uint32_t k = 0, p = p0; k < g.col_cache && p < p1; ++k, p += SELL_ROWS)
+        tlCols[k * TILE + threadIdx.x] = __ldg(&g.col[p]);
+      const S* const from = g.val + size_t(p0 >> 5) * 9 * SELL_ROWS + lane;
+      const uint32_t blocks = min(kept, (p1 - p0 + 31u) >> 5);
+      for (uint32_t k = 0; k < 9u * blocks; ++k) near[k * SELL_ROWS] = __ldg(from + size_t(k) * SELL_ROWS);
+    }
+    __syncthreads();
+    // Block partials alternate between two halves of blk_part by reduction
+    // parity: with one barrier per iteration, a block may write the next
+    // reduction's partials while another still sums the previous one.
+    double* const halves[2] = {s.blk_part + 4 * size_t(it.z), s.blk_part + 4 * (size_t(GANG ? gang.items : G) + it.z)};
+    unsigned int* const arrive = GANG ? &s.counter[b] : &s.sync->arrive;
+    uint32_t reductions = 0;
+    unsigned int bar = 0;
+    Sym<S> Ps = {1, 1, 1, 0, 0, 0};  // the row's preconditioner block, widened where used
+    const auto precondition = [&](V3<double> v) {
+      const Sym<double> P = {double(Ps.xx), double(Ps.yy), double(Ps.zz), double(Ps.xy), double(Ps.xz), double(Ps.yz)};
+      return roundTo<S>(symMul(P, v));
+    };
+    V3<double> x = {0, 0, 0}, r = {0, 0, 0}, rhs = {0, 0, 0};
+    if (live) {
+      const Vec4<S> q0 = s.pre0[row], q1 = s.pre1[row];
+      Ps = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
+      rhs = cvt<double>(xyz(s.right[row]));
+      if (!x0zero) x = cvt<double>(xyz(X[row]));
+    }
+    uint32_t applications = 0;
+    // ---- r = right - A x (anchored rows 0), u = P r, published to vec[1]
+    if (!x0zero) {
+      const V3<double> ax = mine ? sellRow<S, U>(g, slice, lane, X, tlCols, near, kept) : V3<double>{0, 0, 0};
+      if (freeRow) r = rhs - ax;
+      ++applications;
+    } else if (freeRow) {
+      r = rhs;
+    }
+    V3<double> u = precondition(r);
+    Vec4<S>* vec0 = g.vec;
+    Vec4<S>* vec1 = g.vec + g.stride;
+    if (mine) vec1[row] = pack(cvt<S>(u));
+    if (!gangBarrier(arrive, G, s.sync, bar)) return;
+    // ---- w = A u, m = P w published to vec[0], first reduction
+    V3<double> w = mine ? sellRow<S, U>(g, slice, lane, vec1, tlCols, near, kept) : V3<double>{0, 0, 0};
     ++applications;
-  } else if (freeRow) {
-    r = rhs;
-  }
-  V3<double> u = precondition(r);
-  Vec4<S>* vec0 = g.vec;
-  Vec4<S>* vec1 = g.vec + g.stride;
-  if (mine) vec1[row] = pack(cvt<S>(u));
-  if (!countBarrier(s.sync, bar)) return;
-  // ---- w = A u, m = P w published to vec[0], first reduction
-  V3<double> w = mine ? sellRow<S, U>(g, slice, lane, vec1, tlCols) : V3<double>{0, 0, 0};
-  ++applications;
-  V3<double> m = precondition(w);
-  if (mine) vec0[row] = pack(cvt<S>(m));
-  {
-    double v[4] = {dot(r, u), dot(w, u), dot(r, r), live ? dot(rhs, rhs) : 0.0};
-    blockSum<4>(v);
-    if (threadIdx.x == 0)
+    V3<double> m = precondition(w);
+    if (mine) vec0[row] = pack(cvt<S>(m));
+    {
+      double v[4] = {dot(r, u), dot(w, u), dot(r, r), live ? dot(rhs, rhs) : 0.0};
+      blockSum<4>(v);
+      if (threadIdx.x == 0)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) halves[0][k * G + blockIdx.x] = v[k];
-  }
-  if (!countBarrier(s.sync, bar)) return;
-  // n = A m for the first iteration, requested before the block sums so that
-  // their round trip overlaps it (unused if the solve stops here)
-  V3<double> n = mine ? sellRow<S, U>(g, slice, lane, vec0, tlCols) : V3<double>{0, 0, 0};
-  double sums[4];
-  sumBlocksAll<4>(halves[0], sums);
-  ++reductions;
-  double gammaNext = sums[0], delta = sums[1], length = sums[2];
-  const double reference = sqrt(sums[3]);
-  const double floor = fmax(reference, 1.1754943508222875e-38);  // std::numeric_limits<float>::min()
-  const double target = st.tolerance * floor;
-  const double startRes = sqrt(length) / floor;
-  double gamma = 0.0, alpha = 0.0, beta = 0.0;
-  uint32_t taken = 0;
-  V3<double> zv = {0, 0, 0}, qv = {0, 0, 0}, sv = {0, 0, 0}, pv = {0, 0, 0};
-  for (;;) {
-    if (taken >= st.limit || sqrt(length) <= target) break;  // the reference's loop-top test
-    const double b = taken ? gammaNext / gamma : 0.0;
-    const double curvature = taken ? delta - b * gammaNext / alpha : delta;  // p.A p
-    if (!(curvature > 0.0) || !(gammaNext > 0.0)) break;
-    beta = b;
-    alpha = gammaNext / curvature;
-    gamma = gammaNext;
-    if (taken + 1 >= st.limit) {  // the last update the cap allows: no matvec after it
-      pv = u + beta * pv;
+        for (int k = 0; k < 4; ++k) halves[0][k * G + part] = v[k];
+    }
+    if (!gangBarrier(arrive, G, s.sync, bar)) return;
+    // n = A m for the first iteration, requested before the block sums so that
+    // their round trip overlaps it (unused if the solve stops here)
+    V3<double> n = mine ? sellRow<S, U>(g, slice, lane, vec0, tlCols, near, kept) : V3<double>{0, 0, 0};
+    double sums[4];
+    sumBlocksAll<4>(halves[0], sums, G);
+    ++reductions;
+    double gammaNext = sums[0], delta = sums[1], length = sums[2];
+    const double reference = sqrt(sums[3]);
+    const double floor = fmax(reference, 1.1754943508222875e-38);  // std::numeric_limits<float>::min()
+    const double target = st.tolerance * floor;
+    const double startRes = sqrt(length) / floor;
+    double gamma = 0.0, alpha = 0.0, beta = 0.0;
+    uint32_t taken = 0;
+    V3<double> zv = {0, 0, 0}, qv = {0, 0, 0}, sv = {0, 0, 0}, pv = {0, 0, 0};
+    for (;;) {
+      if (taken >= st.limit || sqrt(length) <= target) break;  // the reference's loop-top test
+      const double bl = taken ? gammaNext / gamma : 0.0;
+      const double curvature = taken ? delta - bl * gammaNext / alpha : delta;  // p.A p
+      if (!(curvature > 0.0) || !(gammaNext > 0.0)) break;
+      beta = bl;
+      alpha = gammaNext / curvature;
+      gamma = gammaNext;
+      if (taken + 1 >= st.limit) {  // the last update the cap allows: no matvec after it
+        pv = u + beta * pv;
+        sv = w + beta * sv;
+        x = x + alpha * pv;
+        r = r - alpha * sv;
+        double* mine_part = halves[reductions & 1u];
+        double v[3] = {0.0, 0.0, dot(r, r)};
+        blockSum<3>(v);
+        if (threadIdx.x == 0)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) mine_part[k * G + part] = v[k];
+        if (!gangBarrier(arrive, G, s.sync, bar)) return;
+        double fin[3];
+        sumBlocksAll<3>(mine_part, fin, G);
+        length = fin[2];
+        ++taken;
+        break;
+      }
+      ++applications;  // n = A m of this iteration, computed after the last barrier
+      zv = n + beta * zv;
+      qv = m + beta * qv;
       sv = w + beta * sv;
+      pv = u + beta * pv;
       x = x + alpha * pv;
       r = r - alpha * sv;
-      double* part = halves[reductions & 1u];
-      double v[3] = {0.0, 0.0, dot(r, r)};
-      blockSum<3>(v);
-      if (threadIdx.x == 0)
+      u = u - alpha * qv;
+      w = w - alpha * zv;
+      m = precondition(w);
+      if (mine) ((taken & 1u) ? vec0 : vec1)[row] = pack(cvt<S>(m));
+      double* mine_part = halves[reductions & 1u];
+      {
+        double v[3] = {dot(r, u), dot(w, u), dot(r, r)};
+        blockSum<3>(v);
+        if (threadIdx.x == 0)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) part[k * G + blockIdx.x] = v[k];
-      if (!countBarrier(s.sync, bar)) return;
-      double fin[3];
-      sumBlocksAll<3>(part, fin);
-      length = fin[2];
+          for (int k = 0; k < 3; ++k) mine_part[k * G + part] = v[k];
+      }
+      if (!gangBarrier(arrive, G, s.sync, bar)) return;
+      // n = A m for the next iteration (m just published to vec[(taken + 1) & 1]), with the
+      // block partials requested first so that both round trips overlap
+      if (stagedSums) requestBlockPartials(mine_part, partStage, 3u, G);
+      n = mine ? sellRow<S, U>(g, slice, lane, (taken & 1u) ? vec0 : vec1, tlCols, near, kept) : V3<double>{0, 0, 0};
+      double d[3];
+      if (stagedSums) {
+        cpAsyncWaitAll();
+        __syncthreads();
+        sumStagedBlocks<3>(partStage, d, G);
+      } else {
+        sumBlocksAll<3>(mine_part, d, G);
+      }
+      ++reductions;
+      gammaNext = d[0];
+      delta = d[1];
+      length = d[2];
       ++taken;
-      break;
     }
-    ++applications;  // n = A m of this iteration, computed after the last barrier
-    zv = n + beta * zv;
-    qv = m + beta * qv;
-    sv = w + beta * sv;
-    pv = u + beta * pv;
-    x = x + alpha * pv;
-    r = r - alpha * sv;
-    u = u - alpha * qv;
-    w = w - alpha * zv;
-    m = precondition(w);
-    if (mine) ((taken & 1u) ? vec0 : vec1)[row] = pack(cvt<S>(m));
-    double* part = halves[reductions & 1u];
-    {
-      double v[3] = {dot(r, u), dot(w, u), dot(r, r)};
-      blockSum<3>(v);
-      if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) part[k * G + blockIdx.x] = v[k];
+    if (live) X[row] = pack(cvt<S>(x));
+    if (part == 0 && threadIdx.x == 0) {
+      const double residual = sqrt(length);
+      CgBodyDev c;
+      c.squared = gamma;
+      c.target = target;
+      c.floor = floor;
+      c.length = length;
+      c.stride = alpha;
+      c.blend = beta;
+      c.start_res = startRes;
+      c.rel_res = residual / floor;
+      c.taken = taken;
+      c.done = 1u;
+      c.pad0 = c.pad1 = 0;
+      s.cg[b] = c;
+      CgReportDev rep = s.cgrep[b];
+      rep.iterations += taken;
+      rep.capped += (taken == st.limit && residual > target) ? 1u : 0u;
+      rep.applications += applications;
+      rep.solves += 1u;
+      rep.tangent_iterations += tangent ? taken : 0u;
+      rep.worst_rel = fmax(rep.worst_rel, c.rel_res);
+      if (rep.pass_solves == 0u) rep.pass_start = c.start_res;
+      rep.pass_end = c.rel_res;
+      rep.pass_iterations += c.taken;
+      rep.pass_solves += 1u;
+      s.cgrep[b] = rep;
     }
-    if (!countBarrier(s.sync, bar)) return;
-    // n = A m for the next iteration (m just published to vec[(taken + 1) & 1]), with the
-    // block partials requested first so that both round trips overlap
-    if (stagedSums) requestBlockPartials(part, partStage, 3u);
-    n = mine ? sellRow<S, U>(g, slice, lane, (taken & 1u) ? vec0 : vec1, tlCols) : V3<double>{0, 0, 0};
-    double d[3];
-    if (stagedSums) {
-      cpAsyncWaitAll();
-      __syncthreads();
-      sumStagedBlocks<3>(partStage, d);
-    } else {
-      sumBlocksAll<3>(part, d);
-    }
-    ++reductions;
-    gammaNext = d[0];
-    delta = d[1];
-    length = d[2];
-    ++taken;
-  }
-  if (live) X[row] = pack(cvt<S>(x));
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const double residual = sqrt(length);
-    CgBodyDev c;
-    c.squared = gamma;
-    c.target = target;
-    c.floor = floor;
-    c.length = length;
-    c.stride = alpha;
-    c.blend = beta;
-    c.start_res = startRes;
-    c.rel_res = residual / floor;
-    c.taken = taken;
-    c.done = 1u;
-    c.pad0 = c.pad1 = 0;
-    s.cg[0] = c;
-    CgReportDev rep = s.cgrep[0];
-    rep.iterations += taken;
-    rep.capped += (taken == st.limit && residual > target) ? 1u : 0u;
-    rep.applications += applications;
-    rep.solves += 1u;
-    rep.tangent_iterations += tangent ? taken : 0u;
-    rep.worst_rel = fmax(rep.worst_rel, c.rel_res);
-    if (rep.pass_solves == 0u) rep.pass_start = c.start_res;
-    rep.pass_end = c.rel_res;
-    rep.pass_iterations += c.taken;
-    rep.pass_solves += 1u;
-    s.cgrep[0] = rep;
   }
 }
 

@@ -227,6 +227,7 @@ struct HostBody {
   double restCentre[3] = {0.0, 0.0, 0.0};  // mass-weighted rest centre (of the stored rest positions)
   double mass = 0.0;
   // floats (solver.cc:2964-2971): no anchored node and the rigid split on
+  double reach = 0.0;  // expected PCG iterations of a solve, up to a factor: the cells a step's wave crosses
   bool floats(uint32_t split) const { return split != TL_RIGID_SPLIT_OFF && !anyAnchored; }
 };
 
@@ -377,7 +378,9 @@ struct System final : SystemBase {
   uint32_t batchU() const { return tuneRowGroup ? tuneRowGroup : BATCH_ROW_GROUP; }
   int batchBlocks() const { return tuneBatchBlocks ? int(tuneBatchBlocks) : BATCH_BLOCKS; }
   const void* sellKernel() const {
-    return sellU() == 2u ? (const void*)kPcgSell<S, 2> : (const void*)kPcgSell<S, 4>;
+    const bool two = sellU() == 2u;
+    if (B > 1) return two ? (const void*)kPcgSell<S, true, 2> : (const void*)kPcgSell<S, true, 4>;
+    return two ? (const void*)kPcgSell<S, false, 2> : (const void*)kPcgSell<S, false, 4>;
   }
   const void* batchKernel(bool twoPhase) const {
     const bool u4 = batchU() == 4u, b3 = batchBlocks() == 3;
@@ -744,6 +747,25 @@ struct System final : SystemBase {
         fAnch.assign(d.anchored, d.anchored + d.nodes);
         fMass.assign(d.node_mass, d.node_mass + d.nodes);
       }
+      {  // a solve iterates about as often as a wave crosses cells in a frame (1/60 s), at most the body's own
+        double youngs = 0.0, density = 0.0, volume = 0.0, lo[3], hi[3];
+        for (uint32_t l = 0; l < d.lanes; ++l) youngs = std::max(youngs, d.materials[l].youngs_modulus);
+        for (uint32_t t = 0; t < d.tets; ++t) {
+          volume += d.volume[t];
+          if (d.element_youngs) youngs = std::max(youngs, d.element_youngs[t]);
+        }
+        density = volume > 0.0 ? h.mass / volume : 0.0;
+        for (int k = 0; k < 3; ++k) lo[k] = hi[k] = d.nodes ? d.rest_positions[k] : 0.0;
+        for (uint32_t n = 0; n < d.nodes; ++n)
+          for (int k = 0; k < 3; ++k) {
+            lo[k] = std::min(lo[k], d.rest_positions[3 * size_t(n) + k]);
+            hi[k] = std::max(hi[k], d.rest_positions[3 * size_t(n) + k]);
+          }
+        const double across = std::sqrt((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
+                                        (hi[2] - lo[2]) * (hi[2] - lo[2]));
+        const double wave = density > 0.0 ? std::sqrt(youngs / density) / 60.0 : 0.0;
+        h.reach = volume > 0.0 ? std::min(wave, across) / std::cbrt(volume / double(d.tets)) : 0.0;
+      }
       for (uint32_t t = d.tets; t < bd.elem_tile_end * TILE - bd.elem_begin; ++t) {
         const uint32_t e = bd.elem_begin + t;
         hTet[e] = make_uint4(bd.node_begin, bd.node_begin, bd.node_begin, bd.node_begin);
@@ -921,16 +943,27 @@ struct System final : SystemBase {
     sellVal.zero(st);  // padding blocks stay zero; kSellAssemble writes the others
     sellVec.alloc(size_t(2) * sellStride);
     sellVec.zero(st);
-    for (const void* fn : {(const void*)kPcgSell<S, 2>, (const void*)kPcgSell<S, 4>})
-      TL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sellColBytes())));
-    sellPerSmOf[0] = occupancyOf((const void*)kPcgSell<S, 2>, sellColBytes());
-    sellPerSmOf[1] = occupancyOf((const void*)kPcgSell<S, 4>, sellColBytes());
+    // the most slots in shared memory that cost no residency: 74 KB of a block's blocks, 8 slots in FP32 and 4 in
+    // FP64 (of 15 on a Kuhn lattice), where the columns leave room for it
+    const uint32_t held = tuneRowGroup;
+    int limit = 0;
+    TL_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    const auto perSmOf = [&](uint32_t u) {
+      tuneRowGroup = u;
+      // the attribute is the kernel's, shared by every system: the most any of them may ask for
+      cudaFuncAttributes fa;
+      TL_CUDA(cudaFuncGetAttributes(&fa, sellKernel()));
+      TL_CUDA(cudaFuncSetAttribute(sellKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, limit - int(fa.sharedSizeBytes)));
+      return occupancyOf(sellKernel(), sellColBytes());
+    };
+    sellKept = 0;
+    const int bare[2] = {perSmOf(2u), perSmOf(4u)};
+    for (sellKept = 32u / uint32_t(sizeof(S)); sellKept > 0 && (perSmOf(2u) < bare[0] || perSmOf(4u) < bare[1]);) sellKept -= 4u;
+    sellPerSmOf[0] = perSmOf(2u);
+    sellPerSmOf[1] = perSmOf(4u);
+    tuneRowGroup = held;
     sellPerSm = sellPerSmOf[sellU() == 4u ? 1 : 0];
-    // kPcgSell writes four partials per block into one of two halves
-    {
-      const size_t most = size_t(8) * std::max(sellPerSmOf[0], sellPerSmOf[1]) * ctx->sms;
-      if (most > blkPart.count) blkPart.alloc(most);
-    }
+    buildGang();
     // kPcgBatchSell: every batch, and single bodies whose rows exceed one per thread of kPcgSell's grid
     sellP2.alloc(Vp);
     sellP2.zero(st);
@@ -1029,7 +1062,11 @@ struct System final : SystemBase {
   bool clusterForm() const {
     return sellReady && cluster.kernel && (solverForm == TL_SOLVER_AUTO || solverForm == TL_SOLVER_ASSEMBLED);
   }
-  size_t sellColBytes() const { return size_t(sellColCache) * TILE * sizeof(uint32_t); }
+  // Shared memory of kPcgSell: its first columns and the blocks of its first slots.
+  uint32_t sellKept = 0;
+  size_t sellColBytes() const {
+    return size_t(sellColCache) * TILE * sizeof(uint32_t) + size_t(sellKept) * 9 * TILE * sizeof(S);
+  }
   void assembleSell(const Sys<S>& s, const SellDev<S>& g, unsigned blocks, int idx, bool damp, bool tangent,
                     uint32_t pass) {
     if (idx) {
@@ -1047,6 +1084,7 @@ struct System final : SystemBase {
     SellDev<S> g;
     g.upper_count = sellUpperCount;
     g.col_cache = sellColCache;
+    g.kept = sellKept;
     g.urec = sellUrec.ptr;
     g.rows = sellRows;
     g.slices = sellSlices;
@@ -1073,14 +1111,52 @@ struct System final : SystemBase {
            solverForm == TL_SOLVER_ASSEMBLED_PIPELINED || bodyHost[0].elem_end >= SELL_AUTO_MIN_TETS;
   }
   int sellGrid() const {
-    if (B != 1 || sellPerSm < 1 || !assembledForm()) return 0;
-    const int full = std::min<int>(sellPerSm * ctx->sms, int(sellSlices));
-    const int capped = tuneBlocksPerSm ? std::min<int>(std::min<int>(sellPerSm, int(tuneBlocksPerSm)) * ctx->sms,
-                                                       int(sellSlices))
-                                       : full;
-    const auto fits = [&](int g) { return g > 0 && uint64_t(sellSlices) <= uint64_t(g) * SELL_SLICES_PER_BLOCK; };
-    if (fits(capped)) return capped;
-    return fits(full) ? full : 0;
+    if (sellPerSm < 1 || !assembledForm() || gangGrid == 0) return 0;
+    if (B != 1 && solverForm != TL_SOLVER_AUTO && solverForm != TL_SOLVER_ASSEMBLED) return 0;
+    return gangGrid;
+  }
+  // The items of kPcgSell: each body over enough blocks for one row per thread, and over more, in proportion to
+  // its rows, while the resident grid has blocks to spare.  gangGrid stays 0 when a body does not fit the grid.
+  int gangGrid = 0;
+  uint32_t gangItems = 0;
+  DevBuf<uint4> gangItem;
+  DevBuf<uint2> gangBody;
+  void buildGang() {
+    gangGrid = 0;
+    if (sellPerSm < 1) return;
+    std::vector<uint32_t> slices(B), order(B);
+    uint64_t total = 0;
+    for (uint32_t b = 0; b < B; ++b) {
+      slices[b] = std::max(1u, (bodyHost[b].node_end - bodyHost[b].node_begin + SELL_ROWS - 1) / SELL_ROWS);
+      total += slices[b];
+      order[b] = b;
+    }
+    const uint32_t most = *std::max_element(slices.begin(), slices.end());
+    const auto fits = [&](int g) { return uint64_t(most) <= uint64_t(g) * SELL_SLICES_PER_BLOCK; };
+    int grid = (tuneBlocksPerSm ? std::min<int>(sellPerSm, int(tuneBlocksPerSm)) : sellPerSm) * ctx->sms;
+    if (!fits(grid)) grid = sellPerSm * ctx->sms;
+    if (!fits(grid)) return;
+    // the bodies that iterate longest first, so that no long one starts last (96 uneven bodies: 15.4 ms of PCG per
+    // frame against 18.6 with the most rows first)
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t l, uint32_t r) { return hb[l].reach > hb[r].reach; });
+    std::vector<uint4> item;
+    std::vector<uint2> body(B);
+    for (uint32_t b : order) {
+      body[b] = make_uint2(bodyHost[b].node_begin / SELL_ROWS, slices[b]);
+      const uint32_t least = (slices[b] + SELL_SLICES_PER_BLOCK - 1) / SELL_SLICES_PER_BLOCK;
+      const uint32_t parts = std::max(least, std::min(slices[b], uint32_t(uint64_t(slices[b]) * grid / total)));
+      const uint32_t first = uint32_t(item.size());
+      for (uint32_t q = 0; q < parts; ++q) item.push_back(make_uint4(b, q, first, parts));
+    }
+    gangItems = uint32_t(item.size());
+    gangItem.alloc(item.size());
+    gangItem.upload(item.data(), item.size(), st);
+    gangBody.alloc(B);
+    gangBody.upload(body.data(), B, st);
+    // each item's partials, four values in each of two halves
+    if (size_t(8) * gangItems > blkPart.count) blkPart.alloc(size_t(8) * gangItems);
+    TL_CUDA(cudaStreamSynchronize(st));
+    gangGrid = std::min<int>(grid, int(gangItems));
   }
 
   // Two-level assembly structures: per element tile the distinct nodes it
@@ -1511,6 +1587,7 @@ struct System final : SystemBase {
     const bool damp = hasDamping && idx == 0;
     const bool inCluster = clusterForm();
     const int sellG = inCluster ? 0 : sellGrid();
+    GangDev gang{gangItems, gangItem.ptr, gangBody.ptr};
     if (inCluster) {  // single body that fits a cluster
       SellDev<S> g = sellView();
       const unsigned blocks = (sellUpperCount + TILE - 1) / TILE;
@@ -1537,7 +1614,7 @@ struct System final : SystemBase {
         mark(1, false);
         mark(2, true);
       }
-      void* args[] = {&s, &g, &X, &xz, &tg};
+      void* args[] = {&s, &g, &gang, &X, &ps, &xz, &tg};
       TL_CUDA(cudaLaunchCooperativeKernel(sellKernel(), dim3(sellG), dim3(TILE), args, sellColBytes(), st));
     } else if (B == 1) {  // single body, element by element: two-level assembly, per-block partials
       if (profiling) mark(2, true);
@@ -2322,7 +2399,11 @@ struct System final : SystemBase {
   static constexpr uint32_t OPEN_LAUNCHES = 4;  // openStep's kernels
   std::vector<std::pair<int, size_t>> graphEv;  // event pairs recorded by the captured graph
 
-  void setSolver(uint32_t form) override { solverForm = form; }
+  void setSolver(uint32_t form) override {
+    solverForm = form;
+    if (graphExec) cudaGraphExecDestroy(graphExec);  // the captured launches are the old form's
+    graphExec = nullptr;
+  }
   void expireWait(int32_t solve) override { expireSolve = solve; }
   void setFlowLimits(uint32_t b, uint32_t lane, double crushStress, double crushLimit, double plasticMax) override {
     if (b >= B || lane >= hb[b].lanes) throw StatusError{TL_ERR_ARG, "no such body or material lane"};
@@ -2357,6 +2438,7 @@ struct System final : SystemBase {
   void tune(uint32_t blocksPerSm, uint32_t graph) override {
     tuneBlocksPerSm = blocksPerSm;
     tuneGraph = graph != 0u;
+    if (sellReady) buildGang();
     if (graphExec) cudaGraphExecDestroy(graphExec);
     graphExec = nullptr;
     graphBroken = false;
@@ -2376,6 +2458,7 @@ struct System final : SystemBase {
       batchSellPerSm = occupancyOf(batchKernel(true), 0);
       batchPipePerSm = occupancyOf(batchKernel(false), 0);
       if (batchSellPerSm < 1 || batchPipePerSm < 1) throw StatusError{TL_ERR_CUDA, "shape cannot be resident"};
+      buildGang();
     }
     if (graphExec) cudaGraphExecDestroy(graphExec);  // the captured launches hold the old kernels
     graphExec = nullptr;
