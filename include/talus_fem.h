@@ -238,7 +238,13 @@ int32_t tl_system_set_solver(tl_system* system, uint32_t form);
  * device inside the PCG launch (kPcgFactor).  Needs a one-body system with
  * the assembled operator available and the corotated law on the small-strain
  * path (with or without stiffness damping, whose blocks the factor holds):
- * TL_ERR_UNSUPPORTED otherwise.  enable = 0 drops the state. */
+ * TL_ERR_UNSUPPORTED otherwise.  enable = 0 drops the state.  The factor is
+ * applied through its explicit inverse (kPcgInverse; 0.5 GB of device memory
+ * for 10,000 nodes, 16 GB for 70,000) while that takes at most 24 GB;
+ * enable = TL_FACTOR_LEAN solves with the factor itself (kPcgFactor), which
+ * takes a fifth of the memory or less and 14 times as long or more.  Both
+ * apply the same factor; they differ in rounding. */
+#define TL_FACTOR_LEAN 2u
 int32_t tl_system_use_factor(tl_system* system, uint32_t enable, uint32_t factor_budget);
 
 /* SolverStats (factor.h:28-38), the SystemFactor's size (factor.h:50-62) and

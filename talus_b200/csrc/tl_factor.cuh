@@ -12,7 +12,11 @@
 // Kernels:
 //   kFactorFrame  (one block) the body rotation: polar of the mass-weighted
 //                 correlation of the positions now with the factor's
-//   kPcgFactor    persistent cooperative PCG in the reference's order with
+//   kFactorInverse, kPcgInverse  the inverse of L, and the persistent
+//                 cooperative PCG that applies the factor through it (the
+//                 default)
+//   kPcgFactor    the same PCG with the factor itself (the lean form): in the
+//                 reference's order with
 //                 the factor as preconditioner, operator = the assembled block
 //                 matrix of kSellAssemble.  The two triangular solves of each
 //                 application run inside the launch over the supernodes of the
@@ -519,6 +523,334 @@ __global__ void __launch_bounds__(TILE) kPcgFactor(Sys<S> s, SellDev<S> g, Facto
     c.pad1 = apps;                                               // factor applications
     s.cg[0] = c;
     *f.epoch = epoch0 + apps;
+  }
+}
+
+// ------------------------------------------------- the explicit inverse ----
+// A triangular solve over the supernodes is a chain: 0.3 ms for 1,377 nodes
+// however little it moves, since every row waits for the rows before it.  The
+// dissection keeps L^-1 sparse: row i of it reaches over the rows of its
+// supernode's subtree only, which are contiguous in the order, [first_i, i].
+// So X = L^-1 is kept explicitly, three dense scalar rows per node (17 MB for
+// 1,377 nodes, 513 MB for 9,537, beside 6 and 109 MB of L), and an application
+// is two matvecs without any order among their rows, y = X b and w = X^T y,
+// bound by X's bytes in L2 or HBM.  A step of the 6,144-tet yielding block takes
+// 2.0 ms for 27 (42 iterations), of a 49,152-tet one 18 for 277 (55).
+struct InverseDev {
+  double* x;               // X: node row i's three scalar rows, each 3 (i - first_i + 1) long
+  const uint64_t* off;     // [nodes] start of a node's rows
+  const uint32_t* first;   // [nodes] first row of the node's supernode's subtree
+  uint32_t long_rows, short_rows;
+  const uint32_t* row;     // [long_rows + short_rows] free rows, longest first
+  uint32_t groups, chunks;
+  const uint4* group;      // [groups] columns of w one block makes: first column, its supernode's end, start in anc,
+                           // ancestor rows << 4 | columns; most rows first
+  const uint4* chunk;      // [chunks] the same of kFactorInverse, ancestor rows << 6 | columns
+  const uint32_t* anc;     // rows of each supernode's ancestors, ascending
+  double* b;               // [3 nodes] right side in factor order
+  double* y;               // [3 nodes]
+};
+constexpr uint32_t INVERSE_GROUP = 10;       // nodes: 30 columns, a lane each
+constexpr uint32_t INVERSE_CHUNK = 32;       // nodes of a kFactorInverse block
+constexpr uint32_t INVERSE_T = 3 * INVERSE_CHUNK;
+constexpr uint32_t INVERSE_LONG = 3 * 256;   // scalar columns from which a row takes a whole block
+
+// X from L: a thread per scalar column j, which is the solve L x = e_j over the
+// rows on the path from j's supernode to the root,
+//   x_i = -L_ii^-1 sum_k L_ik x_k, k on the path.
+// The columns are independent, and the threads of a block share the path and
+// the blocks of L; what a thread reads of X it wrote itself.  Once per factor,
+// and small beside the host's part of it: under 2 of 35 ms for 1,377 nodes,
+// 0.15 of 1.4 s for 9,537, where X's rows are read back from L2 once per row
+// that follows.
+static __global__ void __launch_bounds__(INVERSE_T) kFactorInverse(FactorDev f, InverseDev v) {
+  // the entries of a piece of a row of L that lie on the path: column k, place in L, X_k's rows (start less its first
+  // column's offset, length)
+  __shared__ uint32_t listK[INVERSE_T + 4], listAt[INVERSE_T + 4], listLen[INVERSE_T + 4], listCount[INVERSE_T / 32];
+  __shared__ int64_t listX[INVERSE_T + 4];
+  const uint4 c = v.chunk[blockIdx.x];
+  const uint32_t j0 = c.x, end = c.y, columns = c.w & 63u, rows = (end - j0) + (c.w >> 6);
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t j = j0 + threadIdx.x / 3u, comp = threadIdx.x % 3u;
+  const bool active = threadIdx.x < 3u * columns;
+  double* const column = v.x + 3u * size_t(j) + comp;
+  for (uint32_t t = 0; t < rows; ++t) {
+    const uint32_t i = t < end - j0 ? j0 + t : __ldg(&v.anc[c.z + t - (end - j0)]);
+    double acc[3] = {0.0, 0.0, 0.0};
+    const uint32_t q1 = __ldg(&f.row_start[i + 1]);
+    for (uint32_t q0 = __ldg(&f.row_start[i]); q0 < q1; q0 += INVERSE_T) {
+      const uint32_t q = q0 + threadIdx.x, k = q < q1 ? __ldg(&f.row_col[q]) : 0u;
+      const uint32_t f0 = q < q1 ? __ldg(&v.first[k]) : 0u;
+      const bool on = q < q1 && k >= j0 && (k < end || f0 <= j0);
+      const uint32_t ballot = __ballot_sync(0xffffffffu, on);
+      if (lane == 0) listCount[warp] = __popc(ballot);
+      __syncthreads();
+      uint32_t at = __popc(ballot & ((1u << lane) - 1u)), count = 0;
+      for (uint32_t w = 0; w < INVERSE_T / 32; ++w) {
+        if (w < warp) at += listCount[w];
+        count += listCount[w];
+      }
+      if (on) {
+        listK[at] = k;
+        listAt[at] = q;
+        listLen[at] = 3u * (k - f0 + 1u);
+        listX[at] = int64_t(__ldg(&v.off[k])) - 3 * int64_t(f0);
+      }
+      __syncthreads();
+      if (active) {
+        constexpr uint32_t U = 4;  // entries whose loads are issued together
+        for (uint32_t n = 0; n < count; n += U) {
+          double x[U][3], L[U][9];
+#pragma unroll
+          for (uint32_t u = 0; u < U; ++u) {
+            const bool here = n + u < count && listK[n + u] >= j;  // X_kj is 0 for k < j
+            const uint32_t m = n + u < count ? n + u : n;
+            const double* const xk = column + listX[m];
+            const double* const Lk = f.row_blk + size_t(9) * listAt[m];
+#pragma unroll
+            for (uint32_t r = 0; r < 3; ++r) x[u][r] = here ? xk[size_t(r) * listLen[m]] : 0.0;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) L[u][e] = __ldg(Lk + e);
+          }
+#pragma unroll
+          for (uint32_t u = 0; u < U; ++u)
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+              acc[r] = fma(L[u][3 * r], x[u][0], fma(L[u][3 * r + 1], x[u][1], fma(L[u][3 * r + 2], x[u][2], acc[r])));
+        }
+      }
+      __syncthreads();
+    }
+    if (!active || i < j) continue;
+    const double* const D = f.diag_inv + size_t(9) * i;
+    const uint32_t f0 = __ldg(&v.first[i]), len = 3u * (i - f0 + 1u);
+    double* const xi = column + (int64_t(__ldg(&v.off[i])) - 3 * int64_t(f0));
+#pragma unroll
+    for (uint32_t r = 0; r < 3; ++r) {
+      const double d[3] = {__ldg(D + 3 * r), __ldg(D + 3 * r + 1), __ldg(D + 3 * r + 2)};
+      xi[size_t(r) * len] = i == j ? d[comp] : -(d[0] * acc[0] + d[1] * acc[1] + d[2] * acc[2]);
+    }
+  }
+}
+
+// Sums over the warp of three values, in every lane, level by level so that the chains overlap.
+__device__ __forceinline__ void warpSums3(double (&a)[3]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    double t[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) t[r] = __shfl_xor_sync(0xffffffffu, a[r], o);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) a[r] += t[r];
+  }
+}
+
+// y = X b: a block per long row, then a warp per short one.
+__device__ __forceinline__ void inverseForward(const InverseDev& v) {
+  __shared__ double part[2][TILE / 32][3];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, G = gridDim.x;
+  const auto row = [&](uint32_t i, uint32_t from, uint32_t by, double (&a)[3]) {
+    const uint32_t f0 = __ldg(&v.first[i]), len = 3u * (i - f0 + 1u);
+    const double* const x = v.x + __ldg(&v.off[i]);
+    const double* const b = v.b + 3u * size_t(f0);
+    a[0] = a[1] = a[2] = 0.0;
+#pragma unroll 4
+    for (uint32_t k = from; k < len; k += by) {
+      const double bk = __ldcg(b + k);
+      a[0] = fma(__ldg(x + k), bk, a[0]);
+      a[1] = fma(__ldg(x + len + k), bk, a[1]);
+      a[2] = fma(__ldg(x + 2u * size_t(len) + k), bk, a[2]);
+    }
+    warpSums3(a);
+  };
+  double a[3];
+  uint32_t half = 0;
+  for (uint32_t t = blockIdx.x; t < v.long_rows; t += G, half ^= 1u) {
+    const uint32_t i = __ldg(&v.row[t]);
+    row(i, threadIdx.x, TILE, a);
+    if (lane < 3u) part[half][warp][lane] = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];
+    __syncthreads();
+    if (threadIdx.x < 3u) {
+      double sum = 0.0;
+#pragma unroll
+      for (int w = 0; w < TILE / 32; ++w) sum += part[half][w][threadIdx.x];
+      v.y[3u * size_t(i) + threadIdx.x] = sum;
+    }
+  }
+  // the short rows from the last warp on, away from the blocks with one more long row
+  const uint32_t warps = G * (TILE / 32u);
+  for (uint32_t t = warps - 1u - (blockIdx.x * (TILE / 32u) + warp); t < v.short_rows; t += warps) {
+    const uint32_t i = __ldg(&v.row[v.long_rows + t]);
+    row(i, lane, 32u, a);
+    if (lane < 3u) v.y[3u * size_t(i) + lane] = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];
+  }
+}
+
+// w = X^T y, ten nodes a block: lane c of a warp is scalar column c, and the
+// warps share the rows that reach it (the supernode's own from the group on,
+// then its ancestors').  done(node in factor order, w) runs in a lane per node.
+template <class Done>
+__device__ __forceinline__ void inverseBackward(const InverseDev& v, Done done) {
+  __shared__ double part[2][TILE / 32][32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t half = 0;
+  for (uint32_t t = blockIdx.x; t < v.groups; t += gridDim.x, half ^= 1u) {
+    const uint4 g = __ldg(&v.group[t]);
+    const uint32_t j0 = g.x, own = g.y - j0, rows = own + (g.w >> 4), columns = 3u * (g.w & 15u);
+    const bool active = lane < columns;
+    double acc = 0.0;
+#pragma unroll 4
+    for (uint32_t k = warp; k < rows; k += TILE / 32u) {
+      const uint32_t i = k < own ? j0 + k : __ldg(&v.anc[g.z + k - own]);
+      const uint32_t f0 = __ldg(&v.first[i]), len = 3u * (i - f0 + 1u), col = 3u * (j0 - f0) + lane;
+      const double* const x = v.x + __ldg(&v.off[i]) + col;
+      const double* const y = v.y + 3u * size_t(i);
+      const bool here = active && col < len;  // a row of the group itself ends at its own column
+      const double x0 = here ? __ldg(x) : 0.0, x1 = here ? __ldg(x + len) : 0.0, x2 = here ? __ldg(x + 2u * size_t(len)) : 0.0;
+      acc = fma(x0, __ldcg(y), fma(x1, __ldcg(y + 1), fma(x2, __ldcg(y + 2), acc)));
+    }
+    part[half][warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0) {
+      double sum = 0.0;
+#pragma unroll
+      for (int w = 0; w < TILE / 32; ++w) sum += part[half][w][lane];
+      const uint32_t n = min(lane, 9u);
+      const V3<double> w = {__shfl_sync(0xffffffffu, sum, 3 * n), __shfl_sync(0xffffffffu, sum, 3 * n + 1),
+                            __shfl_sync(0xffffffffu, sum, 3 * n + 2)};
+      if (lane < (g.w & 15u)) done(j0 + lane, w);
+    }
+  }
+}
+
+// kPcgFactor with the explicit inverse: the same order, tests and roundings,
+// the direction formed with the matvec that reads it (two buffers in turn), so
+// four grid barriers an iteration.
+template <class S>
+__global__ void __launch_bounds__(TILE, 2) kPcgInverse(Sys<S> s, SellDev<S> g, FactorDev f, InverseDev v, Vec4<S>* X,
+                                                    Vec4<S>* R, Vec4<S>* D, Vec4<S>* D2, Vec4<S>* Q, Vec4<S>* Z,
+                                                    uint32_t x0zero, uint32_t limit) {
+  const uint32_t warps = gridDim.x * (TILE / 32u), gw = blockIdx.x * (TILE / 32u) + (threadIdx.x >> 5);
+  const uint32_t lane = threadIdx.x & 31u;
+  const BodyStepDev st = s.step[0];
+  g.col_cache = 0;  // columns from global memory
+  M3<S> frame;
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) frame.m[i][j] = S(__ldcg(&f.frame[3 * i + j]));
+  unsigned int bar = 0;
+  uint32_t h = 0, apps = 0;
+  auto forRows = [&](auto&& fn) {
+    for (uint32_t slice = gw; slice < g.slices; slice += warps) {
+      const uint32_t row = slice * SELL_ROWS + lane;
+      fn(slice, row, row < g.rows && !s.anch[row], row < g.rows);
+    }
+  };
+  // the residual of a row, and its place in the factor's frame and order (applyFactor)
+  const auto residual = [&](uint32_t row, V3<S> r) {
+    R[row] = pack(r);
+    const V3<double> t = cvt<double>(mulT(frame, r));
+    double* const b = v.b + 3u * size_t(__ldg(&f.iperm[row]));
+    b[0] = t.x;
+    b[1] = t.y;
+    b[2] = t.z;
+  };
+  // z = frame X^T X frame^T r (anchored rows keep their zero); r.z and r.r of the rows made here
+  const auto condition = [&](double& rz, double& rr) -> bool {
+    inverseForward(v);
+    ++apps;
+    if (!countBarrier(s.sync, bar)) return false;
+    rz = rr = 0.0;
+    inverseBackward(v, [&](uint32_t at, V3<double> w) {
+      const uint32_t row = __ldg(&f.perm[at]);
+      const V3<S> z = mul(frame, V3<S>{S(w.x), S(w.y), S(w.z)});
+      Z[row] = pack(z);
+      const V3<double> r = cvt<double>(xyz(ld4cg(&R[row]))), zd = cvt<double>(z);
+      rz += dot(r, zd);
+      rr += dot(r, r);
+    });
+    return true;
+  };
+  // ---- r = right - A x (anchored rows 0), |right|
+  double v0[1] = {0.0};
+  forRows([&](uint32_t slice, uint32_t row, bool freeRow, bool live) {
+    V3<double> r = {0, 0, 0};
+    const V3<double> rhs = live ? cvt<double>(xyz(s.right[row])) : V3<double>{0, 0, 0};
+    if (x0zero) {
+      if (live) X[row] = Vec4<S>{0, 0, 0, 0};
+      if (freeRow) r = rhs;
+    } else {
+      const V3<double> ax = sellRowOf<S, Ld4cg<S>, sellRowGroup<S>(), false>(g, slice, lane, ld4cgOf(X), nullptr);
+      if (freeRow) r = rhs - ax;
+    }
+    if (live) {
+      residual(row, cvt<S>(r));
+      D[row] = Vec4<S>{0, 0, 0, 0};
+      v0[0] += dot(rhs, rhs);
+    }
+  });
+  double refSq[1];
+  if (!gridSum<1>(v0, f.part, h, s.sync, bar, refSq)) return;
+  const double reference = sqrt(refSq[0]);
+  double rz = 0.0, rr = 0.0;
+  if (!condition(rz, rr)) return;
+  double v1[2] = {rz, rr}, s1[2];
+  if (!gridSum<2>(v1, f.part, h, s.sync, bar, s1)) return;
+  double squared = s1[0], length = s1[1];
+  const double floor = fmax(reference, 1.1754943508222875e-38);  // std::numeric_limits<float>::min()
+  const double target = st.tolerance * floor;
+  const double startRes = sqrt(length) / floor;
+  double stride = 0.0, blend = 0.0;
+  uint32_t taken = 0;
+  for (uint32_t iteration = 0; iteration != limit; ++iteration) {
+    if (sqrt(length) <= target) break;
+    const Vec4<S>* const before = (iteration & 1u) ? D2 : D;
+    Vec4<S>* const now = (iteration & 1u) ? D : D2;
+    const auto direction = [&](uint32_t c) {
+      return pack(cvt<S>(cvt<double>(xyz(ld4cg(&Z[c]))) + blend * cvt<double>(xyz(ld4cg(&before[c])))));
+    };
+    double vc[1] = {0.0}, curv[1];
+    forRows([&](uint32_t slice, uint32_t row, bool freeRow, bool live) {
+      const V3<double> q = sellRowOf<S, decltype(direction), sellRowGroup<S>(), false>(g, slice, lane, direction, nullptr);
+      if (!live) return;
+      const V3<S> qs = freeRow ? cvt<S>(q) : V3<S>{0, 0, 0};
+      const Vec4<S> d = direction(row);
+      now[row] = d;
+      Q[row] = pack(qs);
+      vc[0] += dot(cvt<double>(xyz(d)), cvt<double>(qs));
+    });
+    if (!gridSum<1>(vc, f.part, h, s.sync, bar, curv)) return;
+    if (!(curv[0] > 0.0) || !(squared > 0.0)) break;
+    stride = squared / curv[0];
+    forRows([&](uint32_t, uint32_t row, bool, bool live) {
+      if (!live) return;
+      X[row] = pack(cvt<S>(cvt<double>(xyz(X[row])) + stride * cvt<double>(xyz(now[row]))));
+      residual(row, cvt<S>(cvt<double>(xyz(R[row])) - stride * cvt<double>(xyz(Q[row]))));
+    });
+    if (!countBarrier(s.sync, bar)) return;
+    if (!condition(rz, rr)) return;
+    double vn[2] = {rz, rr}, sn[2];
+    if (!gridSum<2>(vn, f.part, h, s.sync, bar, sn)) return;
+    blend = sn[0] / squared;
+    squared = sn[0];
+    length = sn[1];
+    ++taken;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const double residualNorm = sqrt(length);
+    CgBodyDev c;
+    c.squared = squared;
+    c.target = target;
+    c.floor = floor;
+    c.length = length;
+    c.stride = stride;
+    c.blend = blend;
+    c.start_res = startRes;
+    c.rel_res = residualNorm / floor;
+    c.taken = taken;
+    c.done = 1u;
+    c.pad0 = (taken == limit && residualNorm > target) ? 1u : 0u;  // capped
+    c.pad1 = apps;                                                   // factor applications
+    s.cg[0] = c;
   }
 }
 

@@ -448,4 +448,62 @@ struct BlockFactor {
   }
 };
 
+// Layout of X = L^-1 and the work lists of its two matvecs (tl_factor.cuh,
+// InverseDev).  Row i of X reaches over [first_i, i], the rows of its
+// supernode's subtree up to itself; anchored rows have none and are left out.
+struct InversePlan {
+  uint64_t doubles = 0;                // of X
+  std::vector<uint32_t> first;         // [nodes]
+  std::vector<uint64_t> off;           // [nodes]
+  std::vector<uint32_t> rows;          // free rows, longest first
+  uint32_t longRows = 0;               // of them, the rows of at least `longest` scalar columns
+  std::vector<uint32_t> anc;           // rows of each supernode's ancestors, ascending
+  std::vector<uint32_t> group, chunk;  // [4 each] first column, end of its supernode, start in anc, ancestor rows
+                                       // << 4 (group) or << 6 (chunk) | columns
+};
+
+inline InversePlan planInverse(const BlockFactor& f, const uint8_t* anchored, uint32_t groupNodes, uint32_t chunkNodes,
+                               uint32_t longest) {
+  InversePlan p;
+  const uint32_t V = f.nodes;
+  const size_t S = f.snParent.size();
+  p.first.assign(V, 0u);
+  p.off.assign(V, 0u);
+  std::vector<uint32_t> reach(S);  // first row of each supernode's subtree; children come before parents
+  for (size_t q = 0; q < S; ++q) {
+    reach[q] = f.snStart[q];
+    for (int c = 0; c < 2; ++c)
+      if (f.snChild[2 * q + c] >= 0) reach[q] = std::min(reach[q], reach[f.snChild[2 * q + c]]);
+  }
+  std::vector<std::pair<uint32_t, std::vector<uint32_t>>> groups, chunks;  // (rows on the path, record)
+  for (size_t q = 0; q < S; ++q) {
+    const uint32_t b = f.snStart[q], e = f.snStart[q + 1];
+    if (b == e || anchored[f.perm[b]]) continue;
+    for (uint32_t i = b; i < e; ++i) {
+      p.first[i] = reach[q];
+      p.off[i] = p.doubles;
+      p.doubles += uint64_t(9) * (i - reach[q] + 1u);
+      p.rows.push_back(i);
+    }
+    const uint32_t at = uint32_t(p.anc.size());
+    for (int32_t a = f.snParent[q]; a >= 0; a = f.snParent[a])
+      for (uint32_t i = f.snStart[a]; i < f.snStart[a + 1]; ++i) p.anc.push_back(i);
+    const uint32_t above = uint32_t(p.anc.size()) - at;
+    for (uint32_t j = b; j < e; j += groupNodes)
+      groups.push_back({e - j + above, {j, e, at, above << 4 | std::min(groupNodes, e - j)}});
+    for (uint32_t j = b; j < e; j += chunkNodes)
+      chunks.push_back({e - j + above, {j, e, at, above << 6 | std::min(chunkNodes, e - j)}});
+  }
+  std::stable_sort(p.rows.begin(), p.rows.end(),
+                   [&](uint32_t l, uint32_t r) { return l - p.first[l] > r - p.first[r]; });
+  while (p.longRows < p.rows.size() && 3u * (p.rows[p.longRows] - p.first[p.rows[p.longRows]] + 1u) >= longest) ++p.longRows;
+  const auto inOrder = [](auto& list, std::vector<uint32_t>& out) {  // most rows first
+    std::stable_sort(list.begin(), list.end(), [](const auto& l, const auto& r) { return l.first > r.first; });
+    for (const auto& g : list) out.insert(out.end(), g.second.begin(), g.second.end());
+  };
+  inOrder(groups, p.group);
+  inOrder(chunks, p.chunk);
+  return p;
+}
+
 }  // namespace tl

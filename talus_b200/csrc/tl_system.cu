@@ -1706,8 +1706,36 @@ struct System final : SystemBase {
   DevBuf<int32_t> dfSnChild, dfSnParent;
   DevBuf<double> dfRowBlk, dfColBlk, dfDiagInv, dfFrame, dfPart;
   DevBuf<Vec4<double>> dfY, dfW, dfRef, dfRhs;
-  DevBuf<Vec4<S>> dfR, dfD, dfQ, dfZ, dfRestart;
-  int factorPerSm = 0;
+  DevBuf<Vec4<S>> dfR, dfD, dfD2, dfQ, dfZ, dfRestart;
+  int factorPerSm = 0, inversePerSm = 0;
+  // X = L^-1 is kept explicitly (kPcgInverse) while it takes at most INVERSE_MAX bytes and the caller has not asked
+  // for the lean form: 17 MB for 1,377 nodes, 0.5 GB for 9,537, 16 GB for 70,785.  It is the faster one at every size
+  // that was measured (steps of 2.0 against 27 ms, 18 against 277, 37 against 550 at 14,801 nodes); the limit is
+  // what a solver state may take of the device's memory.
+  static constexpr uint64_t INVERSE_MAX = uint64_t(24) << 30;
+  bool fInverse = false, fLean = false;
+  uint32_t fLongRows = 0, fShortRows = 0, fGroups = 0, fChunks = 0;
+  DevBuf<double> dfX, dfB, dfYs;
+  DevBuf<uint64_t> dfOff;
+  DevBuf<uint32_t> dfFirst, dfRows, dfAnc;
+  DevBuf<uint4> dfGroup, dfChunk;
+  InverseDev inverseView() {
+    InverseDev v;
+    v.x = dfX.ptr;
+    v.off = dfOff.ptr;
+    v.first = dfFirst.ptr;
+    v.long_rows = fLongRows;
+    v.short_rows = fShortRows;
+    v.row = dfRows.ptr;
+    v.groups = fGroups;
+    v.chunks = fChunks;
+    v.group = dfGroup.ptr;
+    v.chunk = dfChunk.ptr;
+    v.anc = dfAnc.ptr;
+    v.b = dfB.ptr;
+    v.y = dfYs.ptr;
+    return v;
+  }
 
   void useFactor(uint32_t enable, uint32_t budget) override {
     if (!enable) {
@@ -1718,13 +1746,17 @@ struct System final : SystemBase {
     if (!sellReady) throw StatusError{TL_ERR_UNSUPPORTED, "the factored PCG needs the assembled operator"};
     if (hencky) throw StatusError{TL_ERR_UNSUPPORTED, "the factor is made for the small-strain path"};
     factorOn = true;
+    if (fLean != (enable == TL_FACTOR_LEAN)) fHost.analyzed = false;
+    fLean = enable == TL_FACTOR_LEAN;
     factorBudget = budget;
     fHost.ready = false;
     fStats = tl_factor_stats{};
     fMean = 0.0f;
     if (!factorPerSm) {
       TL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&factorPerSm, kPcgFactor<S>, TILE, 0));
-      if (factorPerSm < 1) throw StatusError{TL_ERR_UNSUPPORTED, "the factored PCG grid cannot be resident"};
+      inversePerSm = occupancyOf((const void*)kPcgInverse<S>, 0);
+      if (factorPerSm < 1 || inversePerSm < 1)
+        throw StatusError{TL_ERR_UNSUPPORTED, "the factored PCG grid cannot be resident"};
     }
   }
   void factorStats(tl_factor_stats* out) override {
@@ -1791,29 +1823,61 @@ struct System final : SystemBase {
       put(dfIperm, fHost.iperm);
       put(dfRowStart, fHost.rowStart);
       put(dfRowCol, fHost.rowCol);
-      put(dfColStart, fHost.colStart);
-      put(dfColRow, fHost.colRow);
-      put(dfSnStart, fHost.snStart);
-      put(dfRowSplit, fHost.rowSplit);
-      put(dfColSplit, fHost.colSplit);
-      auto puti = [&](DevBuf<int32_t>& d, const std::vector<int32_t>& v) {
-        d.alloc(std::max<size_t>(v.size(), 1));
-        d.upload(v.data(), v.size(), st);
-      };
-      puti(dfSnChild, fHost.snChild);
-      puti(dfSnParent, fHost.snParent);
+      dfX.alloc(0);
+      const InversePlan plan = planInverse(fHost, fAnch.data(), INVERSE_GROUP, INVERSE_CHUNK, INVERSE_LONG);
+      fInverse = !fLean && plan.doubles * sizeof(double) <= INVERSE_MAX;
+      if (fInverse && cudaMalloc(&dfX.ptr, std::max<uint64_t>(plan.doubles, 1) * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        dfX.ptr = nullptr;
+        fInverse = false;
+      }
       dfRowBlk.alloc(std::max<size_t>(size_t(9) * fHost.rowCol.size(), 1));
-      dfColBlk.alloc(std::max<size_t>(size_t(9) * fHost.rowCol.size(), 1));
       dfDiagInv.alloc(size_t(9) * std::max<uint32_t>(V, 1));
-      dfY.alloc(std::max<uint32_t>(V, 1));
-      dfW.alloc(std::max<uint32_t>(V, 1));
-      dfRhs.alloc(std::max<uint32_t>(V, 1));
-      dfFlags.alloc(size_t(2) * std::max<size_t>(fHost.snParent.size(), 1));
-      dfFlags.zero(st);
+      if (fInverse) {
+        fLongRows = plan.longRows;
+        fShortRows = uint32_t(plan.rows.size()) - plan.longRows;
+        fGroups = uint32_t(plan.group.size() / 4);
+        fChunks = uint32_t(plan.chunk.size() / 4);
+        put(dfFirst, plan.first);
+        put(dfRows, plan.rows);
+        put(dfAnc, plan.anc);
+        dfOff.alloc(std::max<size_t>(plan.off.size(), 1));
+        dfOff.upload(plan.off.data(), plan.off.size(), st);
+        const auto records = [&](DevBuf<uint4>& d, const std::vector<uint32_t>& v) {
+          d.alloc(std::max<size_t>(v.size() / 4, 1));
+          d.upload(reinterpret_cast<const uint4*>(v.data()), v.size() / 4, st);
+        };
+        records(dfGroup, plan.group);
+        records(dfChunk, plan.chunk);
+        dfB.alloc(size_t(3) * std::max<uint32_t>(V, 1));
+        dfB.zero(st);
+        dfYs.alloc(size_t(3) * std::max<uint32_t>(V, 1));
+        dfYs.zero(st);
+        dfD2.alloc(Vp);
+        dfD2.zero(st);
+      } else {
+        put(dfColStart, fHost.colStart);
+        put(dfColRow, fHost.colRow);
+        put(dfSnStart, fHost.snStart);
+        put(dfRowSplit, fHost.rowSplit);
+        put(dfColSplit, fHost.colSplit);
+        auto puti = [&](DevBuf<int32_t>& d, const std::vector<int32_t>& v) {
+          d.alloc(std::max<size_t>(v.size(), 1));
+          d.upload(v.data(), v.size(), st);
+        };
+        puti(dfSnChild, fHost.snChild);
+        puti(dfSnParent, fHost.snParent);
+        dfColBlk.alloc(std::max<size_t>(size_t(9) * fHost.rowCol.size(), 1));
+        dfY.alloc(std::max<uint32_t>(V, 1));
+        dfW.alloc(std::max<uint32_t>(V, 1));
+        dfRhs.alloc(std::max<uint32_t>(V, 1));
+        dfFlags.alloc(size_t(2) * std::max<size_t>(fHost.snParent.size(), 1));
+        dfFlags.zero(st);
+      }
       dfTicket.alloc(4);
       dfTicket.zero(st);
       dfFrame.alloc(9);
-      dfPart.alloc(size_t(8) * factorPerSm * ctx->sms);
+      dfPart.alloc(size_t(8) * std::max(factorPerSm, inversePerSm) * ctx->sms);
       dfRef.alloc(size_t(V) + 1);
       for (DevBuf<Vec4<S>>* b : {&dfR, &dfD, &dfQ, &dfZ, &dfRestart}) {
         b->alloc(Vp);
@@ -1839,8 +1903,13 @@ struct System final : SystemBase {
     }
     if (fHost.factor(fAnch.data(), fTets, blocks, diag)) {
       dfRowBlk.upload(fHost.rowBlk.data(), fHost.rowBlk.size(), st);
-      dfColBlk.upload(fHost.colBlk.data(), fHost.colBlk.size(), st);
       dfDiagInv.upload(fHost.diagInv.data(), fHost.diagInv.size(), st);
+      if (!fInverse) {
+        dfColBlk.upload(fHost.colBlk.data(), fHost.colBlk.size(), st);
+      } else if (fChunks) {
+        kFactorInverse<<<fChunks, INVERSE_T, 0, st>>>(factorView(), inverseView());
+        check();
+      }
     }
     ++fStats.generation;
     fStep = step;
@@ -1868,11 +1937,18 @@ struct System final : SystemBase {
     Sys<S> s = view();
     SellDev<S> g = sellView();
     FactorDev f = factorView();
-    Vec4<S>*R = dfR.ptr, *D = dfD.ptr, *Q = dfQ.ptr, *Z = dfZ.ptr;
+    Vec4<S>*R = dfR.ptr, *D = dfD.ptr, *D2 = dfD2.ptr, *Q = dfQ.ptr, *Z = dfZ.ptr;
     uint32_t xz = x0zero ? 1u : 0u, lim = limit;
-    void* args[] = {&s, &g, &f, &X, &R, &D, &Q, &Z, &xz, &lim};
-    TL_CUDA(cudaLaunchCooperativeKernel((const void*)kPcgFactor<S>, dim3(factorPerSm * ctx->sms), dim3(TILE), args,
-                                        0, st));
+    if (fInverse) {
+      InverseDev v = inverseView();
+      void* args[] = {&s, &g, &f, &v, &X, &R, &D, &D2, &Q, &Z, &xz, &lim};
+      TL_CUDA(cudaLaunchCooperativeKernel((const void*)kPcgInverse<S>, dim3(inversePerSm * ctx->sms),
+                                          dim3(TILE), args, 0, st));
+    } else {
+      void* args[] = {&s, &g, &f, &X, &R, &D, &Q, &Z, &xz, &lim};
+      TL_CUDA(cudaLaunchCooperativeKernel((const void*)kPcgFactor<S>, dim3(factorPerSm * ctx->sms), dim3(TILE), args,
+                                          0, st));
+    }
     ++launches;
     CgBodyDev c;
     TL_CUDA(cudaMemcpyAsync(&c, cg.ptr, sizeof(CgBodyDev), cudaMemcpyDeviceToHost, st));
