@@ -165,7 +165,6 @@ def pcg_bytes_per_iteration(T, V, slots, s_bytes, tangent):
     return a + b + c
 
 
-SELL_AUTO_MIN_TETS = 32768  # smallest body TL_SOLVER_AUTO assembles (talus_b200/csrc/tl_system.cu)
 
 
 def operator_blocks(mesh):
@@ -539,9 +538,9 @@ def run_ours(args, spec, rank, world, dist):
     s_bytes = 4 if precision == tb.FP32_MIXED else 8
     pcg_bytes = 0.0
     assembly = None
-    # the form the system took (TL_SOLVER_AUTO: assembled for a batch and for one body of >= 32,768 tets)
+    # the form the system took (TL_SOLVER_AUTO: assembled)
     form = tune.get("solver", "auto") if tune else "auto"
-    assembled = form != "elementwise" and (B > 1 or form == "assembled" or meshes[0].tets >= SELL_AUTO_MIN_TETS)
+    assembled = form != "elementwise"
     for b, m in enumerate(meshes):
         it, tan = per_body[b, 0], per_body[b, 1]
         if assembled:  # assembled operator (tl_sell.cuh)

@@ -202,10 +202,9 @@ int32_t tl_system_tune_shape(tl_system* system, uint32_t knob, uint32_t value);
  * the 3x3 node blocks once per solve and iterates on that matrix (about 40
  * bytes per nonzero block in FP32, 76 in FP64);
  * TL_SOLVER_ELEMENTWISE always iterates element by element;
- * TL_SOLVER_AUTO (default) is ASSEMBLED for batched systems, for single
- * bodies of up to 5,120 nodes (which then solve inside one thread-block
- * cluster, kPcgCluster, where their rows fit its shared memory) and for single
- * bodies of at least 32,768 tets, ELEMENTWISE for the single bodies between.
+ * TL_SOLVER_AUTO (default) is ASSEMBLED.  A single body of up to 5,120 nodes
+ * then solves inside one thread-block cluster (kPcgCluster) where its rows
+ * fit the cluster's shared memory, others over the whole GPU (kPcgSell).
  * Both forms apply the same operator; they differ in rounding.  On the
  * assembled matrix ASSEMBLED and AUTO iterate each body of a batch with its
  * own group of blocks, in the pipelined order with one barrier per iteration

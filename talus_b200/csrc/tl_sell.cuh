@@ -235,6 +235,14 @@ template <class S> struct Ld4cg {
   __device__ __forceinline__ Vec4<S> operator()(uint32_t c) const { return ld4cg(&v[c]); }
 };
 template <class S> __device__ __forceinline__ Ld4cg<S> ld4cgOf(const Vec4<S>* v) { return Ld4cg<S>{v}; }
+// acc += block x, the block's entries 32 apart in shared memory.
+template <class S>
+__device__ __forceinline__ void sellNear(const S* v, Vec4<S> xin, V3<double>& acc) {
+  const V3<double> x = cvt<double>(xyz(xin));
+  acc.x = fma(double(v[0]), x.x, fma(double(v[32]), x.y, fma(double(v[64]), x.z, acc.x)));
+  acc.y = fma(double(v[96]), x.x, fma(double(v[128]), x.y, fma(double(v[160]), x.z, acc.y)));
+  acc.z = fma(double(v[192]), x.x, fma(double(v[224]), x.y, fma(double(v[256]), x.z, acc.z)));
+}
 // kPcgSell's row: columns from its shared-memory cache, no prefetch, U slots
 // per round trip, the blocks of its first `kept` slots (a multiple of U) from
 // shared memory.
@@ -244,30 +252,25 @@ __device__ __forceinline__ V3<double> sellRow(const SellDev<S>& g, uint32_t slic
   V3<double> acc = {0, 0, 0};
   const uint32_t p1 = __ldg(&g.slice_start[slice + 1]);
   uint32_t p = __ldg(&g.slice_start[slice]) + lane, k = 0;
+  const auto input = [&](uint32_t i) { return ld4cg(&in[sellCol(cols, g.col_cache, k + i, g.col, p + i * SELL_ROWS)]); };
   for (; k < kept && p + (U - 1) * SELL_ROWS < p1; p += U * SELL_ROWS, k += U) {
     Vec4<S> xin[U];
 #pragma unroll
-    for (uint32_t i = 0; i < U; ++i) xin[i] = ld4cg(&in[sellCol(cols, g.col_cache, k + i, g.col, p + i * SELL_ROWS)]);
+    for (uint32_t i = 0; i < U; ++i) xin[i] = input(i);
 #pragma unroll
-    for (uint32_t i = 0; i < U; ++i) {
-      const S* const v = near + size_t(k + i) * 9 * SELL_ROWS;
-      const V3<double> x = cvt<double>(xyz(xin[i]));
-      acc.x = fma(double(v[0]), x.x, fma(double(v[32]), x.y, fma(double(v[64]), x.z, acc.x)));
-      acc.y = fma(double(v[96]), x.x, fma(double(v[128]), x.y, fma(double(v[160]), x.z, acc.y)));
-      acc.z = fma(double(v[192]), x.x, fma(double(v[224]), x.y, fma(double(v[256]), x.z, acc.z)));
-    }
+    for (uint32_t i = 0; i < U; ++i) sellNear(near + size_t(k + i) * 9 * SELL_ROWS, xin[i], acc);
   }
   for (; p + (U - 1) * SELL_ROWS < p1; p += U * SELL_ROWS, k += U) {
-    uint32_t c[U];
-#pragma unroll
-    for (uint32_t i = 0; i < U; ++i) c[i] = sellCol(cols, g.col_cache, k + i, g.col, p + i * SELL_ROWS);
     Vec4<S> xin[U];
 #pragma unroll
-    for (uint32_t i = 0; i < U; ++i) xin[i] = ld4cg(&in[c[i]]);
+    for (uint32_t i = 0; i < U; ++i) xin[i] = input(i);
 #pragma unroll
     for (uint32_t i = 0; i < U; ++i) sellSlot(g, p + i * SELL_ROWS, lane, xin[i], acc);
   }
-  for (; p < p1; p += SELL_ROWS, ++k) sellSlot(g, p, lane, ld4cg(&in[sellCol(cols, g.col_cache, k, g.col, p)]), acc);
+  for (; p < p1; p += SELL_ROWS, ++k) {
+    if (k < kept) sellNear(near + size_t(k) * 9 * SELL_ROWS, input(0), acc);
+    else sellSlot(g, p, lane, input(0), acc);
+  }
   return acc;
 }
 // Column slots per round trip of the assembled matvec rows (a launch shape
@@ -353,10 +356,11 @@ template <class S> __device__ __forceinline__ V3<double> roundTo(V3<double> v) {
 // The blocks of a row's first `kept` column slots stay in shared memory for the
 // solve: 8 of 15 in FP32, 4 in FP64, as far as two blocks per SM leave room.
 // An SM's matvec reads 400 KB (FP32) to 830 KB through a 64-byte-a-clock port,
-// so this takes 5% off a single body's iteration (9.0 -> 8.7 us at 393,216
-// tets) and 32% off an FP64 batch, whose bodies in work (82 MB) also stop
+// so this takes 3-5% off a single body's iteration (9.0 -> 8.7 us at 393,216
+// tets), all 15 slots with one block per SM 13% (11,424 rows, FP32-mixed: 7.5
+// -> 6.4 us, half of it the barrier of fewer blocks), and 32% off an FP64 batch, whose bodies in work (82 MB) also stop
 // falling out of L2; 8% off an FP32-mixed one.
-template <class S, bool GANG, uint32_t U = sellRowGroup<S>()>
+template <class S, bool GANG, uint32_t U>
 __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, GangDev gang, Vec4<S>* X, uint32_t pass, uint32_t x0zero, uint32_t tangent) {
   const uint32_t lane = threadIdx.x & 31u;
   // [col_cache][TILE] the first columns of each thread's row, then [TILE / 32][g.kept][9][32] its warp's first blocks

@@ -238,6 +238,7 @@ struct tl_ctx {
   cudaStream_t stream = nullptr;
   int sms = 0;
   std::string last_error;
+  int sellShared[2][2] = {{-1, -1}, {-1, -1}};   // dynamic shared memory a kPcgSell block may take, [FP64][batch]
   int clusterFits[2][2] = {{-1, -1}, {-1, -1}};  // whether the device runs kPcgCluster, [FP64][K - 1]; -1: not asked yet
 };
 
@@ -401,7 +402,6 @@ struct System final : SystemBase {
   DevBuf<uint4> sellUrec;  // kSellAssemble's per-block records
   uint32_t sellUpperCount = 0, sellColCache = 0;
   static constexpr uint32_t SELL_COL_CACHE_MAX = 32;  // column slots per thread in kPcgSell's shared memory
-  static constexpr uint32_t SELL_AUTO_MIN_TETS = 32768;  // TL_SOLVER_AUTO: smallest body that is assembled
   DevBuf<S> sellVal;
   DevBuf<Vec4<S>> sellVec;
   int pcg1PerSm[2][2] = {{0, 0}, {0, 0}};   // resident blocks per SM, [law][tangent]
@@ -943,24 +943,43 @@ struct System final : SystemBase {
     sellVal.zero(st);  // padding blocks stay zero; kSellAssemble writes the others
     sellVec.alloc(size_t(2) * sellStride);
     sellVec.zero(st);
-    // the most slots in shared memory that cost no residency: 74 KB of a block's blocks, 8 slots in FP32 and 4 in
-    // FP64 (of 15 on a Kuhn lattice), where the columns leave room for it
+    // Slots whose blocks stay in shared memory.  A body (or batch) that needs two blocks per SM: as many as cost no
+    // residency, 8 in FP32 and 4 in FP64 (of 15 on a Kuhn lattice).  One body that fits a block per SM gets one, which
+    // makes its barrier the cheaper (11,424 rows: 6.7 us an iteration with 148 blocks for 7.5 with 296; 30,576 rows in
+    // FP64 8.2 for 8.8), and then all that an SM holds.
+    sellAlone = B == 1 && (sellSlices + SELL_SLICES_PER_BLOCK - 1) / SELL_SLICES_PER_BLOCK <= uint32_t(ctx->sms);
     const uint32_t held = tuneRowGroup;
-    int limit = 0;
-    TL_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    int& sellShared = ctx->sellShared[sizeof(S) == 8 ? 1 : 0][B > 1 ? 1 : 0];  // dynamic shared memory kPcgSell may take
     const auto perSmOf = [&](uint32_t u) {
       tuneRowGroup = u;
-      // the attribute is the kernel's, shared by every system: the most any of them may ask for
-      cudaFuncAttributes fa;
-      TL_CUDA(cudaFuncGetAttributes(&fa, sellKernel()));
-      TL_CUDA(cudaFuncSetAttribute(sellKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, limit - int(fa.sharedSizeBytes)));
       return occupancyOf(sellKernel(), sellColBytes());
     };
+    if (sellShared < 0) {  // once per context: the attribute is the kernels', so it covers every system
+      int limit = 0;
+      TL_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+      int least = limit;
+      for (uint32_t u : {2u, 4u}) {
+        tuneRowGroup = u;
+        cudaFuncAttributes fa;
+        TL_CUDA(cudaFuncGetAttributes(&fa, sellKernel()));
+        TL_CUDA(cudaFuncSetAttribute(sellKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, limit - int(fa.sharedSizeBytes)));
+        least = std::min(least, limit - int(fa.sharedSizeBytes));
+      }
+      sellShared = least;
+    }
     sellKept = 0;
-    const int bare[2] = {perSmOf(2u), perSmOf(4u)};
-    for (sellKept = 32u / uint32_t(sizeof(S)); sellKept > 0 && (perSmOf(2u) < bare[0] || perSmOf(4u) < bare[1]);) sellKept -= 4u;
-    sellPerSmOf[0] = perSmOf(2u);
-    sellPerSmOf[1] = perSmOf(4u);
+    if (sellAlone) {
+      const size_t room = (size_t(sellShared) - sellColBytes()) / (size_t(9) * TILE * sizeof(S));
+      sellKept = uint32_t(std::min<size_t>((widest + 3u) / 4u, room / 4u)) * 4u;
+      sellPerSmOf[0] = sellPerSmOf[1] = 1;
+    } else {
+      const int bare[2] = {perSmOf(2u), perSmOf(4u)};
+      for (sellKept = 32u / uint32_t(sizeof(S));; sellKept -= 4u) {
+        sellPerSmOf[0] = perSmOf(2u);
+        sellPerSmOf[1] = perSmOf(4u);
+        if (sellKept == 0 || (sellPerSmOf[0] >= bare[0] && sellPerSmOf[1] >= bare[1])) break;
+      }
+    }
     tuneRowGroup = held;
     sellPerSm = sellPerSmOf[sellU() == 4u ? 1 : 0];
     buildGang();
@@ -1064,6 +1083,7 @@ struct System final : SystemBase {
   }
   // Shared memory of kPcgSell: its first columns and the blocks of its first slots.
   uint32_t sellKept = 0;
+  bool sellAlone = false;  // one body that fits a block per SM: its grid is that, with an SM's shared memory
   size_t sellColBytes() const {
     return size_t(sellColCache) * TILE * sizeof(uint32_t) + size_t(sellKept) * 9 * TILE * sizeof(S);
   }
@@ -1098,18 +1118,12 @@ struct System final : SystemBase {
     g.vec = sellVec.ptr;
     return g;
   }
-  // Grid of kPcgSell: the occupancy (capped by tl_system_tune while every
-  // block still has at most one slice per warp), or 0 when the rows do not
-  // fit one per thread.
-  // Whether this system's PCG runs on the assembled matrix.  TL_SOLVER_AUTO
-  // assembles batches, and single bodies large enough for the per-solve
-  // assembly to pay (measured on a B200: element-by-element 17% faster at
-  // 3,072 tets, even at 24,576, assembled 1.6x faster at 393,216).
-  bool assembledForm() const {
-    if (!sellReady || solverForm == TL_SOLVER_ELEMENTWISE) return false;
-    return B > 1 || solverForm == TL_SOLVER_ASSEMBLED || solverForm == TL_SOLVER_ASSEMBLED_TWO_PHASE ||
-           solverForm == TL_SOLVER_ASSEMBLED_PIPELINED || bodyHost[0].elem_end >= SELL_AUTO_MIN_TETS;
-  }
+  // Whether this system's PCG runs on the assembled matrix, which TL_SOLVER_AUTO always chooses: with one block per
+  // SM kPcgSell overtakes the element-by-element kernel for every body past a cluster's (5,202 nodes, a frame: 1.19
+  // against 1.38 ms in FP32-mixed, 1.40 against 1.59 in FP64, the assembly included).
+  bool assembledForm() const { return sellReady && solverForm != TL_SOLVER_ELEMENTWISE; }
+  // Grid of kPcgSell, or 0 where it does not run: a body with more rows than the grid has threads, or a batch in one
+  // of the lockstep orders.
   int sellGrid() const {
     if (sellPerSm < 1 || !assembledForm() || gangGrid == 0) return 0;
     if (B != 1 && solverForm != TL_SOLVER_AUTO && solverForm != TL_SOLVER_ASSEMBLED) return 0;
