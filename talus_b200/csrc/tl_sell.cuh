@@ -68,26 +68,59 @@ template <class S> struct SellDev {
 };
 
 // Block (a, b) of one element's operator, d y_a / d p_b in FP64, where y is
-// the element matvec of elementApply.  Corotated law without damping in
-// closed form: with gh = R g, sigma(e) = k.x tr(e) I + k.y e - k.z (n : e) n
+// the element matvec of elementApply, in closed form.
+// Corotated law: with gh = R g, sigma(e) = k.x tr(e) I + k.y e - k.z (n : e) n
 // and e = sym(p_b gh_b^T),
 //   B_ij = k.x gh_a,i gh_b,j + k.y (delta_ij gh_a.gh_b + gh_b,i gh_a,j) / 2
 //          - k.z (n gh_a)_i (n gh_b)_j.
-// Otherwise the columns are the element operator applied to the three unit
-// vectors at corner b.
+// Neo-Hookean law: dP = k.x dF + k.y dcof + k.z (cof F : dF) cof F for
+// dF = p_b g_b^T, where dcof g_a = p_b x F (g_a x g_b), so
+//   B = k.x g_a.g_b I + k.z (cof F g_a)(cof F g_b)^T - k.y [F (g_a x g_b)]_x.
+// Stiffness damping adds Pi K Pi of the rigid motion's removal Pi, by the
+// strains E_b^j of unit motions less their fit (fittedStrain):
+//   B_ij += a tr E_a^i tr E_b^j + b E_a^i : E_b^j.
+// Bound by FP64 latency and issue.  Against products with the three unit
+// vectors, us a solve with the node assembly: 126 -> 48 FP64 and 50 -> 40 mixed
+// for a damped block of 18,480 tets (671 -> 107 and 123 -> 80 at 162,000), and
+// 58 -> 40 and 36 -> 32 for a neo-Hookean one of 24,576 (188 -> 85 and 59 -> 50).
 // v_i for a run-time corner index, by selects (no local-memory array).
 template <class T>
 __device__ __forceinline__ V3<T> pick(const V3<T>& v0, const V3<T>& v1, const V3<T>& v2, const V3<T>& v3, uint32_t i) {
   return i == 0 ? v0 : i == 1 ? v1 : i == 2 ? v2 : v3;
 }
 
+// The damping share of block (a, b) from the fit kept by kDamping.
+template <class S>
+__device__ __forceinline__ void addDampingBlock(const Sys<S>& s, uint32_t e, const ElementOperator<S>& o, uint32_t a,
+                                                uint32_t b, V3<double> ga, V3<double> gb, double (&acc)[9]) {
+  const auto fit = [&](uint32_t q) { return double(__ldg(s.dfit + size_t(q) * s.Tp + e)); };
+  const V3<double> arm[4] = {{fit(0), fit(1), fit(2)}, {fit(3), fit(4), fit(5)}, {fit(6), fit(7), fit(8)},
+                             {fit(9), fit(10), fit(11)}};
+  const Sym<double> inv = {fit(12), fit(13), fit(14), fit(15), fit(16), fit(17)};
+  const double ca = fit(18), cb = fit(19);
+  const V3<double> gh[4] = {cvt<double>(o.g[0]), cvt<double>(o.g[1]), cvt<double>(o.g[2]), cvt<double>(o.g[3])};
+  V3<double> col[3];
+  armMoment(arm, gh, col);
+  const V3<double> armA = pick(arm[0], arm[1], arm[2], arm[3], a), armB = pick(arm[0], arm[1], arm[2], arm[3], b);
+  const Sym<double> ea[3] = {fittedStrain(inv, col, armA, ga, 0), fittedStrain(inv, col, armA, ga, 1),
+                             fittedStrain(inv, col, armA, ga, 2)};
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const Sym<double> eb = fittedStrain(inv, col, armB, gb, j);
+    const double tr = ca * symTrace(eb);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) acc[3 * i + j] += tr * symTrace(ea[i]) + cb * symContract(ea[i], eb);
+  }
+}
+
 template <class S, int LAW, bool TANGENT, bool DAMP>
 __device__ __forceinline__ void addElementBlock(const Sys<S>& s, uint32_t e, uint32_t a, uint32_t b,
                                                 double (&acc)[9]) {
   const ElementOperator<S> o = loadOperator<S, LAW, TANGENT>(s, e);
-  if constexpr (LAW == 0 && !DAMP) {
-    const V3<double> ga = cvt<double>(pick(o.g[0], o.g[1], o.g[2], o.g[3], a)),
-                     gb = cvt<double>(pick(o.g[0], o.g[1], o.g[2], o.g[3], b));
+  const V3<double> ga = cvt<double>(pick(o.g[0], o.g[1], o.g[2], o.g[3], a)),
+                   gb = cvt<double>(pick(o.g[0], o.g[1], o.g[2], o.g[3], b));
+  const double A[3] = {ga.x, ga.y, ga.z}, Bv[3] = {gb.x, gb.y, gb.z};
+  if constexpr (LAW == 0) {
     const double kx = double(o.k.x), hy = 0.5 * double(o.k.y);
     const double gg = hy * dot(ga, gb);
     V3<double> na = {0, 0, 0}, nb = {0, 0, 0};
@@ -98,27 +131,30 @@ __device__ __forceinline__ void addElementBlock(const Sys<S>& s, uint32_t e, uin
       na = kz * symMul(n, ga);
       nb = symMul(n, gb);
     }
-    const double A[3] = {ga.x, ga.y, ga.z}, Bv[3] = {gb.x, gb.y, gb.z};
     const double NA[3] = {na.x, na.y, na.z}, NB[3] = {nb.x, nb.y, nb.z};
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
       for (int j = 0; j < 3; ++j)
         acc[3 * i + j] += kx * A[i] * Bv[j] + hy * Bv[i] * A[j] + (i == j ? gg : 0.0) - NA[i] * NB[j];
-  } else {
-#pragma unroll 1
-    for (int j = 0; j < 3; ++j) {
-      const V3<S> unit = {S(j == 0), S(j == 1), S(j == 2)}, zero = {0, 0, 0};
-      V3<S> p[4], y[4];
-#pragma unroll
-      for (uint32_t c = 0; c < 4; ++c) p[c] = c == b ? unit : zero;
-      applyOperator<S, LAW, TANGENT>(o, p, y);
-      if (DAMP && LAW == 0) dampingProduct(s, e, o.g, p, y);
-      const V3<S> ya = pick(y[0], y[1], y[2], y[3], a);
-      acc[j] += double(ya.x);
-      acc[3 + j] += double(ya.y);
-      acc[6 + j] += double(ya.z);
+    if constexpr (DAMP) {
+      if (s.dtau[e] != S(0)) addDampingBlock(s, e, o, a, b, ga, gb, acc);
     }
+  } else {
+    M3<double> F;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) F.m[i][j] = double(o.F.m[i][j]);
+    const M3<double> C = cofactor(F);
+    const V3<double> ca = double(o.k.z) * mul(C, ga), cb = mul(C, gb), w = double(o.k.y) * mul(F, cross(ga, gb));
+    const double gg = double(o.k.x) * dot(ga, gb);
+    const double CA[3] = {ca.x, ca.y, ca.z}, CB[3] = {cb.x, cb.y, cb.z};
+    const double turn[9] = {gg, w.z, -w.y, -w.z, gg, w.x, w.y, -w.x, gg};
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc[3 * i + j] += CA[i] * CB[j] + turn[3 * i + j];
   }
 }
 
@@ -131,7 +167,7 @@ __device__ __forceinline__ void addElementBlock(const Sys<S>& s, uint32_t e, uin
 // into the preconditioner) is this operator's.  Padding positions are zero
 // from the build and are never written.
 template <class S, int LAW, bool TANGENT, bool DAMP>
-__global__ void __launch_bounds__(TILE, 4) kSellAssemble(Sys<S> s, SellDev<S> g, uint32_t pass) {
+__global__ void __launch_bounds__(TILE, DAMP ? 2 : 4) kSellAssemble(Sys<S> s, SellDev<S> g, uint32_t pass) {
   const uint32_t i = blockIdx.x * TILE + threadIdx.x;
   if (i >= g.upper_count) return;
   // one record holds what the block needs, so its first contributor's code is requested

@@ -1100,6 +1100,7 @@ struct System final : SystemBase {
       else kSellAssemble<S, 0, false, false><<<blocks, TILE, 0, st>>>(s, g, pass);
     }
   }
+
   SellDev<S> sellView() {
     SellDev<S> g;
     g.upper_count = sellUpperCount;
