@@ -239,7 +239,8 @@ int32_t tl_system_set_solver(tl_system* system, uint32_t form);
  * path (with or without stiffness damping, whose blocks the factor holds):
  * TL_ERR_UNSUPPORTED otherwise.  enable = 0 drops the state.  The factor is
  * applied through its explicit inverse (kPcgInverse; 0.5 GB of device memory
- * for 10,000 nodes, 16 GB for 70,000) while that takes at most 24 GB;
+ * for 10,000 nodes, 16 GB for 70,000) while that takes at most 24 GB and
+ * half of the free device memory;
  * enable = TL_FACTOR_LEAN solves with the factor itself (kPcgFactor), which
  * takes a fifth of the memory or less and 14 times as long or more.  Both
  * apply the same factor; they differ in rounding. */

@@ -16,10 +16,10 @@ through ``System.tune``:
   batched kernels are compiled for (3 registers-richer, or 4).  They change
   only the launch shape; the results are bitwise the same.
 * ``solver``: the PCG operator form (``System.set_solver``): "auto" (the
-  block matrix assembled once per solve, for these workloads), for a batch
-  "assembled-two-phase" (two grid barriers per iteration, fewer bytes) and
-  "assembled-pipelined" (one barrier per iteration, FP64 recurrences), or
-  "elementwise".  The block cap applies to the element-by-element kernels;
+  block matrix assembled once per solve, each body iterated by its own blocks),
+  for a batch also the lockstep orders "assembled-two-phase" (two grid barriers
+  per iteration, fewer bytes) and "assembled-pipelined" (one barrier per
+  iteration, FP64 recurrences), or "elementwise".  The block cap applies to the element-by-element kernels;
   the assembled ones take their own occupancy, so they are timed at 0.
 
 Every candidate starts from the same rest state and runs the same steps, so
@@ -45,6 +45,7 @@ def candidates(bodies: int):
     out = [("elementwise", k, g, 0, 0) for k in (0, 1, 2, 3) for g in graphs]
     if bodies == 1:
         return out + [("auto", 0, False, rg, 0) for rg in (2, 4)]
+    out += [("auto", 0, g, rg, 0) for g in graphs for rg in (2, 4)]
     forms = ["assembled-two-phase", "assembled-pipelined"]
     for form in forms:
         out += [(form, 0, g, 0, 0) for g in graphs]

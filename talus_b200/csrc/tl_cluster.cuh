@@ -141,18 +141,6 @@ __device__ __forceinline__ bool barWait(uint32_t bar, uint32_t parity, GridSyncD
   }
 }
 
-// 1 / a by Newton's iteration on the hardware's estimate (a few ulp), for the
-// one division on an iteration's path; numbers outside the normal range's
-// middle take the division.
-__device__ __forceinline__ double reciprocal(double a) {
-  const double m = fabs(a);
-  if (!(m > 1.0e-290 && m < 1.0e290)) return 1.0 / a;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  y = fma(y, fma(-a, y, 1.0), y);
-  return fma(y, fma(-a, y, 1.0), y);
-}
-
 // Sum over the warp, in every lane.
 __device__ __forceinline__ double warpSum(double v) {
 #pragma unroll
@@ -515,7 +503,7 @@ __global__ void __launch_bounds__(CLUSTER_T, 1)
       rr = warpSum(rr);
       sendPair(ru, rr);
       if (warp == 0 && taken) {
-        inverse = reciprocal(gamma);
+        inverse = 1.0 / gamma;
         ratio *= inverse;
       }
       products();
@@ -534,7 +522,7 @@ __global__ void __launch_bounds__(CLUSTER_T, 1)
           bl = taken ? ru * inverse : 0.0;
           const double pAp = taken ? wu - bl * ru * ratio : wu;
           if (pAp > 0.0 && ru > 0.0) {
-            a = ru * reciprocal(pAp);
+            a = ru / pAp;
             ratio = pAp;
             gamma = ru;
             next2 = 0.0;

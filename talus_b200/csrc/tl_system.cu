@@ -1725,8 +1725,8 @@ struct System final : SystemBase {
   int factorPerSm = 0, inversePerSm = 0;
   // X = L^-1 is kept explicitly (kPcgInverse) while it takes at most INVERSE_MAX bytes and the caller has not asked
   // for the lean form: 17 MB for 1,377 nodes, 0.5 GB for 9,537, 16 GB for 70,785.  It is the faster one at every size
-  // that was measured (steps of 2.0 against 27 ms, 18 against 277, 37 against 550 at 14,801 nodes); the limit is
-  // what a solver state may take of the device's memory.
+  // that was measured (steps of 2.0 against 27 ms, 18 against 277, 37 against 550 at 14,801 nodes); the limit,
+  // and half of the memory that is free, are what a solver state may take of the device's memory.
   static constexpr uint64_t INVERSE_MAX = uint64_t(24) << 30;
   bool fInverse = false, fLean = false;
   uint32_t fLongRows = 0, fShortRows = 0, fGroups = 0, fChunks = 0;
@@ -1840,7 +1840,9 @@ struct System final : SystemBase {
       put(dfRowCol, fHost.rowCol);
       dfX.alloc(0);
       const InversePlan plan = planInverse(fHost, fAnch.data(), INVERSE_GROUP, INVERSE_CHUNK, INVERSE_LONG);
-      fInverse = !fLean && plan.doubles * sizeof(double) <= INVERSE_MAX;
+      size_t idle = 0, whole = 0;
+      TL_CUDA(cudaMemGetInfo(&idle, &whole));
+      fInverse = !fLean && plan.doubles * sizeof(double) <= std::min<uint64_t>(INVERSE_MAX, idle / 2);
       if (fInverse && cudaMalloc(&dfX.ptr, std::max<uint64_t>(plan.doubles, 1) * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         dfX.ptr = nullptr;
