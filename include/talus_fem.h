@@ -189,8 +189,8 @@ int32_t tl_system_tune(tl_system* system, uint32_t pcg_blocks_per_sm, uint32_t g
 /* Launch shape of the assembled-operator PCG, no reference counterpart
  * (chosen by talus_b200/autotune.py); results are bitwise the same for every
  * shape. TL_SHAPE_ROW_GROUP: column slots of a matrix row whose inputs and
- * blocks are requested per round trip, 2 or 4 (0 = the default: 4 in FP32
- * and 2 in FP64, 2 in the lockstep batched orders). TL_SHAPE_BATCH_BLOCKS:
+ * blocks are requested per round trip, 2 or 4 (0 = the default: 4, but
+ * 2 for an FP32-mixed batch and in the lockstep batched orders). TL_SHAPE_BATCH_BLOCKS:
  * resident 256-thread blocks per SM the lockstep batched kernels are compiled
  * for, 3 or 4 (0 = 4). Other values return TL_ERR_ARG. */
 #define TL_SHAPE_ROW_GROUP 0u

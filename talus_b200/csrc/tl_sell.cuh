@@ -309,8 +309,9 @@ __device__ __forceinline__ V3<double> sellRow(const SellDev<S>& g, uint32_t slic
   }
   return acc;
 }
-// Column slots per round trip of the assembled matvec rows (a launch shape
-// tl_system_tune_shape may change): kPcgSell's default, then the batched kernels'.
+// Column slots per round trip of the assembled matvec rows: the factored
+// kernels', then the lockstep kernels' default (a launch shape, as kPcgSell's,
+// that tl_system_tune_shape may change).
 template <class S> __host__ __device__ constexpr uint32_t sellRowGroup() { return sizeof(S) == 4 ? 4u : 2u; }
 constexpr uint32_t BATCH_ROW_GROUP = 2u;
 constexpr int BATCH_BLOCKS = 4;  // resident blocks per SM the batched kernels are compiled for by default

@@ -375,7 +375,9 @@ struct System final : SystemBase {
   // matrix row (0: the kernel's default) and resident blocks per SM of the batched kernels (0: 4)
   uint32_t tuneRowGroup = 0, tuneBatchBlocks = 0;
   int sellPerSmOf[2] = {0, 0};  // kPcgSell with row groups 2 and 4
-  uint32_t sellU() const { return tuneRowGroup ? tuneRowGroup : sellRowGroup<S>(); }
+  // kPcgSell's default: 4 slots a round trip, 2 in an FP32-mixed batch.  512 uneven bodies to 1e-6, a step: FP64 133.5
+  // ms with 4 and 140.8 with 2, FP32-mixed 92.1 and 90.1 (whose matvec has half the bytes to wait for).
+  uint32_t sellU() const { return tuneRowGroup ? tuneRowGroup : sizeof(S) == 4 && B > 1 ? 2u : 4u; }
   uint32_t batchU() const { return tuneRowGroup ? tuneRowGroup : BATCH_ROW_GROUP; }
   int batchBlocks() const { return tuneBatchBlocks ? int(tuneBatchBlocks) : BATCH_BLOCKS; }
   const void* sellKernel() const {
