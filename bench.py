@@ -806,8 +806,8 @@ def solver_state_form(context, cells=(16, 8, 8), warmup=1, steps=4, budget=32):
             out[name].update({"refactor_seconds": st["refactor_seconds"], "factor_nonzeros": st["factor_nonzeros"],
                               "refactor_count": st["refactor_count"], "retries": st["retries"]})
         s.close()
-    out["note"] = ("the factored solves are latency-bound on the elimination tree's longest path "
-                   "(kPcgFactor); the factor is made on the host at the first step")
+    out["note"] = ("the factor is applied through its explicit inverse (kPcgInverse: four grid "
+                   "barriers an iteration); it is made on the host at the first step")
     return out
 
 
