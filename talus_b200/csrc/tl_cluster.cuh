@@ -389,8 +389,9 @@ __global__ void __launch_bounds__(CLUSTER_T, 1)
     // their number.
     double* const red = reinterpret_cast<double*>(tlCluster + lay.red);
     bool timely = true;  // no wait of warp 0 ran out
-    const auto ownersMeet = [&]() {
+    const auto ownersMeet = [&]() {  // lane 0's entries of red are then visible to every owner's lanes
       if (c.owners > 1u) asm volatile("bar.sync 1, %0;" ::"r"(32u * c.owners) : "memory");
+      else __syncwarp();
     };
     const auto sendPair = [&](double a, double bb) {
       if (lane == 0) {

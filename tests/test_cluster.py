@@ -132,3 +132,23 @@ def test_cluster_solves_match_the_elementwise_form(cells, shuffle, precision, to
     assert relative_error(out["auto"][0], out["elementwise"][0], mesh.rest_positions) <= tol
     if precision == tb.FP64:
         assert out["auto"][1] == out["elementwise"][1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells", [(1, 1, 1), (1, 1, 7), (7, 7, 7)])
+@pytest.mark.parametrize("precision", [tb.FP64, tb.FP32_MIXED])
+def test_blocks_of_one_owner_take_the_same_decisions(cells, precision):
+    """Bodies of at most 16 slices: one warp of a block owns its rows, and its lanes each send the block's sums, which
+    lane 0 wrote, to another block.  Every block has to see the same sums, so a repeated solve is bitwise the same."""
+    mesh = tb.box_mesh(cells, voxel=0.1, jitter=0.01, seed=3)
+    mat = tb.PhysicalMaterial(density=1000.0, youngs_modulus=1e7, poissons_ratio=0.3)
+    s = tb.System(mesh, [mat], precision)
+    out = []
+    for _ in range(8):
+        s.set_state(tb.rest_state(mesh))
+        its = [s.step(tb.Settings(tolerance=1e-6, cg_iterations=500), GRAVITY, DT)[0].cg_iterations for _ in range(4)]
+        out.append((its, s.get_state().position))
+    s.close()
+    for its, x in out[1:]:
+        assert its == out[0][0]
+        assert np.array_equal(x, out[0][1])
