@@ -409,6 +409,7 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
   constexpr unsigned SELL_PART_STAGE_BLOCKS = 320;
   __shared__ __align__(16) double partStage[3 * SELL_PART_STAGE_BLOCKS + 2];
   __shared__ uint32_t queued[2];  // two, as a block may pass over an item without a barrier
+  __shared__ int stopped;
   for (uint32_t turn = 0;; ++turn) {
     uint32_t item = blockIdx.x;  // the block's first item, then the queue's
     if (GANG && turn) {
@@ -430,6 +431,9 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
     const bool freeRow = live && !s.anch[row];
     const BodyStepDev st = s.step[b];
     const bool stagedSums = G <= SELL_PART_STAGE_BLOCKS;
+    // a wait that ran out, in this solve or an earlier one of the step, ends the solve: a body of one part meets no
+    // barrier that would look
+    if (threadIdx.x == 0) stopped = *(volatile int*)&s.sync->error;
     if (mine) {
       const uint32_t p0 = __ldg(&g.slice_start[slice]) + lane, p1 = __ldg(&g.slice_start[slice + 1]);
       for (uint32_t k = 0, p = p0; k < g.col_cache && p < p1; ++k, p += SELL_ROWS)
@@ -439,6 +443,7 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
       for (uint32_t k = 0; k < 9u * blocks; ++k) near[k * SELL_ROWS] = __ldg(from + size_t(k) * SELL_ROWS);
     }
     __syncthreads();
+    if (stopped != 0) return;
     // Block partials alternate between two halves of blk_part by reduction
     // parity: with one barrier per iteration, a block may write the next
     // reduction's partials while another still sums the previous one.

@@ -81,3 +81,48 @@ def test_factored_solve_reports_an_expired_wait(solve):
     assert np.isfinite(system.get_state().position).all()
     assert system.factor_stats()["ready"] == 1
     system.close()
+
+
+def _expired_step(system, solve):
+    assert capi.lib().tl_system_expire_wait(system.handle, solve) == capi.TL_OK
+    reports = (tb.StepReport * len(system.meshes))()
+    g = np.asarray(GRAVITY, np.float64)
+    return capi.lib().tl_step(system.handle, C.byref(tb.Settings()._c()), g.ctypes.data, DT, reports)
+
+
+# one body over many blocks of kPcgSell; bodies of one block each; one of several beside one of one
+@pytest.mark.parametrize("cells", [[(16, 16, 17)], [(3, 3, 3), (2, 5, 3), (4, 4, 4)], [(12, 11, 10), (2, 2, 2)]])
+@pytest.mark.parametrize("precision", [tb.FP64, tb.FP32_MIXED])
+def test_every_solve_of_a_step_leaves_after_an_expired_wait(cells, precision):
+    """kPcgSell over one body and over a batch's queue: a wait that ran out before the first solve ends all solves of
+    the step, those of bodies that meet no barrier too, so no acceleration of a body at rest changes.  The next step
+    runs normally."""
+    meshes = [tb.box_mesh(c, voxel=0.1, jitter=0.01, seed=6) for c in cells]
+    mats = [[tb.PhysicalMaterial(density=1000.0, youngs_modulus=1e6, poissons_ratio=0.3)] for _ in meshes]
+    system = tb.System(meshes, mats, precision)
+    for i, m in enumerate(meshes):
+        system.set_state(tb.rest_state(m), i)
+    assert _expired_step(system, 0) == capi.TL_ERR_TIMEOUT
+    for i in range(len(meshes)):
+        assert not system.get_state(i).acceleration.any(), i
+    for i, m in enumerate(meshes):
+        system.set_state(tb.rest_state(m), i)
+    reports = system.step(tb.Settings(), GRAVITY, DT)
+    assert all(r.cg_iterations > 0 for r in reports)
+    for i in range(len(meshes)):
+        assert np.isfinite(system.get_state(i).position).all()
+    system.close()
+
+
+@pytest.mark.parametrize("solve", [0, 2])
+def test_the_lean_factored_solve_reports_an_expired_wait(solve):
+    mesh, mat = elastic_block((4, 4, 4), seed=6)
+    system = tb.System(mesh, [mat], tb.FP64)
+    capi.check(capi.lib().tl_system_use_factor(system.handle, 2, 32), system.context.handle)
+    system.set_state(tb.rest_state(mesh))
+    system.step(tb.Settings(), GRAVITY, DT)
+    assert _expired_step(system, solve) == capi.TL_ERR_TIMEOUT
+    system.set_state(tb.rest_state(mesh))
+    assert system.step(tb.Settings(), GRAVITY, DT)[0].cg_iterations > 0
+    assert system.factor_stats()["ready"] == 1
+    system.close()
