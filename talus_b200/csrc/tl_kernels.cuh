@@ -39,6 +39,10 @@ template <> __device__ __forceinline__ Vec4<double> ld4cg<double>(const Vec4<dou
   const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
   return {a.x, a.y, b.x, b.y};
 }
+__device__ __forceinline__ Packed3 ld4cg(const Packed3* p) {
+  const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p));
+  return {v.x, v.y, v.z, v.w};
+}
 // Read-only (non-coherent cache) loads of data no kernel writes during the launch.
 template <class S> __device__ __forceinline__ Vec4<S> ld4g(const Vec4<S>* p);
 template <> __device__ __forceinline__ Vec4<float> ld4g<float>(const Vec4<float>* p) {

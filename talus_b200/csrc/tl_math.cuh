@@ -5,7 +5,9 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <cfloat>
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 
 #define TL_HD __host__ __device__ __forceinline__
@@ -27,6 +29,34 @@ template <class T> TL_HD V3<T> cross(V3<T> a, V3<T> b) {
   return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
 template <class T, class U> TL_HD V3<T> cvt(V3<U> a) { return {T(a.x), T(a.y), T(a.z)}; }
+
+// Three FP64 values in 16 bytes: the sign, the exponent and 30 bits of the
+// fraction of each, rounded to nearest, the upper words as they are and the 10
+// bits of each lower word together.  Reading one takes five integer
+// operations; a conversion from FP32 costs more and holds 23 bits.
+struct alignas(16) Packed3 {
+  uint32_t x, y, z, low;
+};
+TL_HD uint64_t packedBits(double v) {
+  uint64_t b;
+  memcpy(&b, &v, 8);
+  return fabs(v) <= DBL_MAX ? b + (uint64_t(1) << 21) : b;  // an infinity or NaN keeps its upper word
+}
+TL_HD Packed3 pack3(V3<double> v) {
+  const uint64_t x = packedBits(v.x), y = packedBits(v.y), z = packedBits(v.z);
+  return {uint32_t(x >> 32), uint32_t(y >> 32), uint32_t(z >> 32),
+          (uint32_t(x) >> 22) | (uint32_t(y) >> 22) << 10 | (uint32_t(z) >> 22) << 20};
+}
+TL_HD double fromWords(uint32_t high, uint32_t low) {
+  const uint64_t b = uint64_t(high) << 32 | low;
+  double v;
+  memcpy(&v, &b, 8);
+  return v;
+}
+TL_HD V3<double> unpack3(Packed3 p) {
+  return {fromWords(p.x, p.low << 22), fromWords(p.y, p.low << 12 & 0xffc00000u),
+          fromWords(p.z, p.low << 2 & 0xffc00000u)};
+}
 
 template <class T>
 struct M3 {

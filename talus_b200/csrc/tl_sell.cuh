@@ -28,7 +28,7 @@
 //                  iteration with its matvec, so each iteration needs one grid
 //                  barrier.  Each thread owns one node row and keeps its
 //                  vectors in FP64 registers; only the matvec input is
-//                  published (rounded to S, and used rounded on both sides).
+//                  published (Published<S>, used as rounded on both sides).
 //                  In a batch each body is iterated by just enough blocks,
 //                  which take bodies from a queue.
 //
@@ -48,6 +48,17 @@ namespace tl {
 
 constexpr uint32_t SELL_SLICES_PER_BLOCK = TILE / SELL_ROWS;
 
+// A row's entry of the vector that an iteration of the pipelined kernels
+// publishes for the next matvec.  Their recurrences never form u = P r again
+// between two replacements, so what they add up has to hold more digits than
+// the tolerance asks for: FP64 as it is, and in FP32-mixed 31 significant bits
+// in the 16 bytes that three floats take.
+template <class S> using Published = std::conditional_t<sizeof(S) == 8, Vec4<double>, Packed3>;
+template <class S> __device__ __forceinline__ Published<S> publishedOf(V3<double> v) {
+  if constexpr (sizeof(S) == 8) return pack(v);
+  else return pack3(v);
+}
+
 template <class S> struct SellDev {
   uint32_t rows;                 // one body: its nodes; a batch: every node slot of the system
   uint32_t slices;               // ceil(rows / 32)
@@ -64,7 +75,7 @@ template <class S> struct SellDev {
   const uint4* urec;
   const uint32_t* centry;        // (element << 4) | (row corner << 2) | column corner
   S* val;                        // [positions / 32][9][32]
-  Vec4<S>* vec;                  // [2][stride] published matvec inputs
+  Published<S>* vec;             // [2][stride] published matvec inputs
 };
 
 // Block (a, b) of one element's operator, d y_a / d p_b in FP64, where y is
@@ -204,12 +215,17 @@ __device__ __forceinline__ uint32_t sellCol(const uint32_t* cols, uint32_t cache
   return k < cache ? cols[k * TILE + threadIdx.x] : __ldg(&gcol[p]);
 }
 
+// A matvec input as it is read, in FP64.
+template <class T> __device__ __forceinline__ V3<double> wideOf(const Vec4<T>& v) { return cvt<double>(xyz(v)); }
+__device__ __forceinline__ V3<double> wideOf(const Packed3& v) { return unpack3(v); }
+// v as the published vector holds it.
+template <class S> __device__ __forceinline__ V3<double> roundPublished(V3<double> v) { return wideOf(publishedOf<S>(v)); }
+
 // One column slot of the thread's row: acc += block(p) x.
-template <class S>
-__device__ __forceinline__ void sellSlot(const SellDev<S>& g, uint32_t p, uint32_t lane, Vec4<S> xin,
-                                         V3<double>& acc) {
+template <class S, class V>
+__device__ __forceinline__ void sellSlot(const SellDev<S>& g, uint32_t p, uint32_t lane, V xin, V3<double>& acc) {
   const S* v = g.val + size_t(p >> 5) * 9 * SELL_ROWS + lane;
-  const V3<double> x = cvt<double>(xyz(xin));
+  const V3<double> x = wideOf(xin);
   const double b0 = __ldg(v), b1 = __ldg(v + 32), b2 = __ldg(v + 64), b3 = __ldg(v + 96), b4 = __ldg(v + 128),
                b5 = __ldg(v + 160), b6 = __ldg(v + 192), b7 = __ldg(v + 224), b8 = __ldg(v + 256);
   acc.x = fma(b0, x.x, fma(b1, x.y, fma(b2, x.z, acc.x)));
@@ -236,7 +252,7 @@ __device__ __forceinline__ V3<double> sellRowOf(const SellDev<S>& g, uint32_t sl
     for (uint32_t i = 0; i < U; ++i)
       c[i] = p + i * SELL_ROWS < p1 ? sellCol(cols, g.col_cache, k + i, g.col, p + i * SELL_ROWS) : 0u;
     for (; p + (U - 1) * SELL_ROWS < p1; p += U * SELL_ROWS, k += U) {
-      Vec4<S> xin[U];
+      decltype(in(0u)) xin[U];
 #pragma unroll
       for (uint32_t i = 0; i < U; ++i) xin[i] = in(c[i]);
       const uint32_t pn = p + U * SELL_ROWS;
@@ -255,7 +271,7 @@ __device__ __forceinline__ V3<double> sellRowOf(const SellDev<S>& g, uint32_t sl
       uint32_t c[U];
 #pragma unroll
       for (uint32_t i = 0; i < U; ++i) c[i] = sellCol(cols, g.col_cache, k + i, g.col, p + i * SELL_ROWS);
-      Vec4<S> xin[U];
+      decltype(in(0u)) xin[U];
 #pragma unroll
       for (uint32_t i = 0; i < U; ++i) xin[i] = in(c[i]);
 #pragma unroll
@@ -266,15 +282,16 @@ __device__ __forceinline__ V3<double> sellRowOf(const SellDev<S>& g, uint32_t sl
   return acc;
 }
 // The matvec input read from a vector written during the launch (L2).
-template <class S> struct Ld4cg {
-  const Vec4<S>* v;
-  __device__ __forceinline__ Vec4<S> operator()(uint32_t c) const { return ld4cg(&v[c]); }
+template <class V> struct LdCg {
+  const V* v;
+  __device__ __forceinline__ V operator()(uint32_t c) const { return ld4cg(&v[c]); }
 };
-template <class S> __device__ __forceinline__ Ld4cg<S> ld4cgOf(const Vec4<S>* v) { return Ld4cg<S>{v}; }
+template <class S> using Ld4cg = LdCg<Vec4<S>>;
+template <class V> __device__ __forceinline__ LdCg<V> ld4cgOf(const V* v) { return LdCg<V>{v}; }
 // acc += block x, the block's entries 32 apart in shared memory.
-template <class S>
-__device__ __forceinline__ void sellNear(const S* v, Vec4<S> xin, V3<double>& acc) {
-  const V3<double> x = cvt<double>(xyz(xin));
+template <class S, class V>
+__device__ __forceinline__ void sellNear(const S* v, V xin, V3<double>& acc) {
+  const V3<double> x = wideOf(xin);
   acc.x = fma(double(v[0]), x.x, fma(double(v[32]), x.y, fma(double(v[64]), x.z, acc.x)));
   acc.y = fma(double(v[96]), x.x, fma(double(v[128]), x.y, fma(double(v[160]), x.z, acc.y)));
   acc.z = fma(double(v[192]), x.x, fma(double(v[224]), x.y, fma(double(v[256]), x.z, acc.z)));
@@ -282,22 +299,21 @@ __device__ __forceinline__ void sellNear(const S* v, Vec4<S> xin, V3<double>& ac
 // kPcgSell's row: columns from its shared-memory cache, no prefetch, U slots
 // per round trip, the blocks of its first `kept` slots (a multiple of U) from
 // shared memory.
-template <class S, uint32_t U>
-__device__ __forceinline__ V3<double> sellRow(const SellDev<S>& g, uint32_t slice, uint32_t lane,
-                                              const Vec4<S>* in, const uint32_t* cols, const S* near, uint32_t kept) {
+template <class S, uint32_t U, class V>
+__device__ __forceinline__ V3<double> sellRow(const SellDev<S>& g, uint32_t slice, uint32_t lane, const V* in, const uint32_t* cols, const S* near, uint32_t kept) {
   V3<double> acc = {0, 0, 0};
   const uint32_t p1 = __ldg(&g.slice_start[slice + 1]);
   uint32_t p = __ldg(&g.slice_start[slice]) + lane, k = 0;
   const auto input = [&](uint32_t i) { return ld4cg(&in[sellCol(cols, g.col_cache, k + i, g.col, p + i * SELL_ROWS)]); };
   for (; k < kept && p + (U - 1) * SELL_ROWS < p1; p += U * SELL_ROWS, k += U) {
-    Vec4<S> xin[U];
+    V xin[U];
 #pragma unroll
     for (uint32_t i = 0; i < U; ++i) xin[i] = input(i);
 #pragma unroll
     for (uint32_t i = 0; i < U; ++i) sellNear(near + size_t(k + i) * 9 * SELL_ROWS, xin[i], acc);
   }
   for (; p + (U - 1) * SELL_ROWS < p1; p += U * SELL_ROWS, k += U) {
-    Vec4<S> xin[U];
+    V xin[U];
 #pragma unroll
     for (uint32_t i = 0; i < U; ++i) xin[i] = input(i);
 #pragma unroll
@@ -395,10 +411,31 @@ template <class S> __device__ __forceinline__ V3<double> roundTo(V3<double> v) {
 // An SM's matvec reads 400 KB (FP32) to 830 KB through a 64-byte-a-clock port,
 // so this takes 3-5% off a single body's iteration (9.0 -> 8.7 us at 393,216
 // tets), all 15 slots with one block per SM 13% (11,424 rows, FP32-mixed: 7.5
-// -> 6.4 us, half of it the barrier of fewer blocks), and 32% off an FP64 batch, whose bodies in work (82 MB) also stop
-// falling out of L2; 8% off an FP32-mixed one.
+// -> 6.4 us, half of it the barrier of fewer blocks), and 32% off an FP64
+// batch, whose bodies in work (82 MB) also stop falling out of L2; 8% off an
+// FP32-mixed one.
+//
+// Replacement.  u and q are never formed from r and s again, and w, s and z
+// never from u, p and q, so they keep the rounding of their largest values.
+// Once r.r or r.u has fallen by SELL_FALL from its largest since the last
+// replacement and the target is not reached, all are formed anew: p as it is
+// published, s = A p, u = P r, w = A u, q = P s, z = A q; in FP64 r = right - A x
+// too, whose gap to the carried r the late iterations would not see (in
+// FP32-mixed x is not held to the digits that this would take).  p, gamma and
+// alpha go on.  The fall lies where the default tolerance of 1e-3 does not
+// reach it: 0 replacements a solve there, 1 at 1e-6 and 3 at 1e-11.  Without it,
+// and with m published in FP32, 92 of 576 solves of 96 uneven bodies stopped
+// above 1e-6 in FP32-mixed on the breakdown test, the worst at 1e-3, and a
+// layered body (stiffnesses 1e4 apart) at 0.3; with it none does, and they take
+// as many iterations as the textbook order (34,989 for 35,684 before in a frame
+// of those bodies: 32.0 ms for 32.2; FP64 steps of 166,050 tets take 8.07
+// ms for 7.89, FP32-mixed ones of 393,216 tets 9.5 for 9.8, as unpacking is
+// cheaper than converting).
+// The steps are written out in FP64 and a loop in FP32-mixed, as each spills least.
+constexpr int SELL_FALL = 23 << 20;  // a factor of 2^-23, in the upper word of a double
 template <class S, bool GANG, uint32_t U>
-__global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, GangDev gang, Vec4<S>* X, uint32_t pass, uint32_t x0zero, uint32_t tangent) {
+__global__ void __launch_bounds__(TILE, 2)
+    kPcgSell(Sys<S> s, SellDev<S> g, GangDev gang, Vec4<S>* X, uint32_t pass, uint32_t x0zero, uint32_t tangent) {
   const uint32_t lane = threadIdx.x & 31u;
   // [col_cache][TILE] the first columns of each thread's row, then [TILE / 32][g.kept][9][32] its warp's first blocks
   extern __shared__ __align__(16) uint32_t tlCols[];
@@ -410,6 +447,7 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
   __shared__ __align__(16) double partStage[3 * SELL_PART_STAGE_BLOCKS + 2];
   __shared__ uint32_t queued[2];  // two, as a block may pass over an item without a barrier
   __shared__ int stopped;
+  __shared__ uint32_t extra;  // operator applications of the replacements
   for (uint32_t turn = 0;; ++turn) {
     uint32_t item = blockIdx.x;  // the block's first item, then the queue's
     if (GANG && turn) {
@@ -433,7 +471,10 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
     const bool stagedSums = G <= SELL_PART_STAGE_BLOCKS;
     // a wait that ran out, in this solve or an earlier one of the step, ends the solve: a body of one part meets no
     // barrier that would look
-    if (threadIdx.x == 0) stopped = *(volatile int*)&s.sync->error;
+    if (threadIdx.x == 0) {
+      stopped = *(volatile int*)&s.sync->error;
+      extra = 0u;
+    }
     if (mine) {
       const uint32_t p0 = __ldg(&g.slice_start[slice]) + lane, p1 = __ldg(&g.slice_start[slice + 1]);
       for (uint32_t k = 0, p = p0; k < g.col_cache && p < p1; ++k, p += SELL_ROWS)
@@ -444,17 +485,23 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
     }
     __syncthreads();
     if (stopped != 0) return;
-    // Block partials alternate between two halves of blk_part by reduction
-    // parity: with one barrier per iteration, a block may write the next
-    // reduction's partials while another still sums the previous one.
-    double* const halves[2] = {s.blk_part + 4 * size_t(it.z), s.blk_part + 4 * (size_t(GANG ? gang.items : G) + it.z)};
+    // The published vectors and the block partials alternate between two halves
+    // by the number of barriers passed: what is written before a barrier is read
+    // after it, and until all blocks have passed the next one.
     unsigned int* const arrive = GANG ? &s.counter[b] : &s.sync->arrive;
-    uint32_t reductions = 0;
     unsigned int bar = 0;
+    const auto vec = [&]() { return g.vec + ((bar & 1u) ? size_t(g.stride) : size_t(0)); };
+    const auto partials = [&]() {
+      return s.blk_part + 4 * (size_t((bar & 1u) ? (GANG ? gang.items : G) : 0u) + it.z);
+    };
+    const auto product = [&]() {  // of the vector published before the last barrier
+      return mine ? sellRow<S, U>(g, slice, lane, g.vec + ((bar & 1u) ? size_t(0) : size_t(g.stride)), tlCols, near, kept)
+                  : V3<double>{0, 0, 0};
+    };
     Sym<S> Ps = {1, 1, 1, 0, 0, 0};  // the row's preconditioner block, widened where used
     const auto precondition = [&](V3<double> v) {
       const Sym<double> P = {double(Ps.xx), double(Ps.yy), double(Ps.zz), double(Ps.xy), double(Ps.xz), double(Ps.yz)};
-      return roundTo<S>(symMul(P, v));
+      return roundPublished<S>(symMul(P, v));
     };
     V3<double> x = {0, 0, 0}, r = {0, 0, 0}, rhs = {0, 0, 0};
     if (live) {
@@ -463,85 +510,116 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
       rhs = cvt<double>(xyz(s.right[row]));
       if (!x0zero) x = cvt<double>(xyz(X[row]));
     }
-    uint32_t applications = 0;
-    // ---- r = right - A x (anchored rows 0), u = P r, published to vec[1]
+    // ---- r = right - A x (anchored rows 0), u = P r published
     if (!x0zero) {
       const V3<double> ax = mine ? sellRow<S, U>(g, slice, lane, X, tlCols, near, kept) : V3<double>{0, 0, 0};
       if (freeRow) r = rhs - ax;
-      ++applications;
     } else if (freeRow) {
       r = rhs;
     }
     V3<double> u = precondition(r);
-    Vec4<S>* vec0 = g.vec;
-    Vec4<S>* vec1 = g.vec + g.stride;
-    if (mine) vec1[row] = pack(cvt<S>(u));
+    if (mine) vec()[row] = publishedOf<S>(u);
     if (!gangBarrier(arrive, G, s.sync, bar)) return;
-    // ---- w = A u, m = P w published to vec[0], first reduction
-    V3<double> w = mine ? sellRow<S, U>(g, slice, lane, vec1, tlCols, near, kept) : V3<double>{0, 0, 0};
-    ++applications;
+    // ---- w = A u, m = P w published, first reduction
+    V3<double> w = product();
     V3<double> m = precondition(w);
-    if (mine) vec0[row] = pack(cvt<S>(m));
+    if (mine) vec()[row] = publishedOf<S>(m);
+    const double* part4 = partials();
     {
       double v[4] = {dot(r, u), dot(w, u), dot(r, r), live ? dot(rhs, rhs) : 0.0};
       blockSum<4>(v);
       if (threadIdx.x == 0)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) halves[0][k * G + part] = v[k];
+        for (int k = 0; k < 4; ++k) partials()[k * G + part] = v[k];
     }
     if (!gangBarrier(arrive, G, s.sync, bar)) return;
     // n = A m for the first iteration, requested before the block sums so that
     // their round trip overlaps it (unused if the solve stops here)
-    V3<double> n = mine ? sellRow<S, U>(g, slice, lane, vec0, tlCols, near, kept) : V3<double>{0, 0, 0};
+    V3<double> n = product();
     double sums[4];
-    sumBlocksAll<4>(halves[0], sums, G);
-    ++reductions;
+    sumBlocksAll<4>(part4, sums, G);
     double gammaNext = sums[0], delta = sums[1], length = sums[2];
-    const double reference = sqrt(sums[3]);
-    const double floor = fmax(reference, 1.1754943508222875e-38);  // std::numeric_limits<float>::min()
-    const double target = st.tolerance * floor;
-    const double startRes = sqrt(length) / floor;
+    double target = 0.0;
+    {
+      const double floor = fmax(sqrt(sums[3]), 1.1754943508222875e-38);  // std::numeric_limits<float>::min()
+      target = st.tolerance * floor;
+      if (part == 0 && threadIdx.x == 0) {
+        s.cg[b].floor = floor;
+        s.cg[b].start_res = sqrt(length) / floor;
+      }
+    }
     double gamma = 0.0, alpha = 0.0, beta = 0.0;
     uint32_t taken = 0;
     V3<double> zv = {0, 0, 0}, qv = {0, 0, 0}, sv = {0, 0, 0}, pv = {0, 0, 0};
+    int mostLength = 0, mostGamma = 0;  // upper words of the largest since the last replacement
+    bool fresh = true;                  // no update since then
     for (;;) {
       if (taken >= st.limit || sqrt(length) <= target) break;  // the reference's loop-top test
-      const double bl = taken ? gammaNext / gamma : 0.0;
-      const double curvature = taken ? delta - bl * gammaNext / alpha : delta;  // p.A p
-      if (!(curvature > 0.0) || !(gammaNext > 0.0)) break;
-      beta = bl;
-      alpha = gammaNext / curvature;
-      gamma = gammaNext;
-      if (taken + 1 >= st.limit) {  // the last update the cap allows: no matvec after it
-        pv = u + beta * pv;
+      mostLength = max(fresh ? 0 : mostLength, __double2hiint(length));
+      mostGamma = max(fresh ? 0 : mostGamma, __double2hiint(gammaNext));
+      if (!fresh && (__double2hiint(length) < mostLength - SELL_FALL || __double2hiint(gammaNext) < mostGamma - SELL_FALL)) {
+        constexpr int copies = sizeof(S) == 8 ? 4 : 1;
+        // x (FP64), p, P r and P s published in turn: r = right - A x, s = A p, w = A u, z = A q
+#pragma unroll copies
+        for (uint32_t k = sizeof(S) == 8 ? 0u : 1u; k < 4u; ++k) {
+          const V3<double> v = k == 0u ? x : k == 1u ? roundPublished<S>(pv) : precondition(k == 2u ? r : sv);
+          if (mine) vec()[row] = publishedOf<S>(v);
+          if (!gangBarrier(arrive, G, s.sync, bar)) return;
+          const V3<double> y = product();
+          if (k == 0u) {
+            if (freeRow) r = cvt<double>(xyz(s.right[row])) - y;
+          } else if (k == 1u) {
+            pv = v;
+            sv = y;
+          } else if (k == 2u) {
+            u = v;
+            w = y;
+          } else {
+            qv = v;
+            zv = y;
+          }
+        }
+        if (threadIdx.x == 0) extra += sizeof(S) == 8 ? 4u : 3u;
+        fresh = true;
+      } else {
+        const double bl = taken ? gammaNext / gamma : 0.0;
+        const double curvature = taken ? delta - bl * gammaNext / alpha : delta;  // p.A p
+        if (!(curvature > 0.0) || !(gammaNext > 0.0)) break;
+        beta = bl;
+        alpha = gammaNext / curvature;
+        gamma = gammaNext;
+        if (taken + 1 >= st.limit) {  // the last update the cap allows: no matvec after it
+          pv = u + beta * pv;
+          sv = w + beta * sv;
+          x = x + alpha * pv;
+          r = r - alpha * sv;
+          const double* last = partials();
+          double v[3] = {0.0, 0.0, dot(r, r)};
+          blockSum<3>(v);
+          if (threadIdx.x == 0)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) partials()[k * G + part] = v[k];
+          if (!gangBarrier(arrive, G, s.sync, bar)) return;
+          double fin[3];
+          sumBlocksAll<3>(last, fin, G);
+          length = fin[2];
+          ++taken;
+          break;
+        }
+        zv = n + beta * zv;
+        qv = m + beta * qv;
         sv = w + beta * sv;
+        pv = u + beta * pv;
         x = x + alpha * pv;
         r = r - alpha * sv;
-        double* mine_part = halves[reductions & 1u];
-        double v[3] = {0.0, 0.0, dot(r, r)};
-        blockSum<3>(v);
-        if (threadIdx.x == 0)
-#pragma unroll
-          for (int k = 0; k < 3; ++k) mine_part[k * G + part] = v[k];
-        if (!gangBarrier(arrive, G, s.sync, bar)) return;
-        double fin[3];
-        sumBlocksAll<3>(mine_part, fin, G);
-        length = fin[2];
+        u = u - alpha * qv;
+        w = w - alpha * zv;
         ++taken;
-        break;
+        fresh = false;
       }
-      ++applications;  // n = A m of this iteration, computed after the last barrier
-      zv = n + beta * zv;
-      qv = m + beta * qv;
-      sv = w + beta * sv;
-      pv = u + beta * pv;
-      x = x + alpha * pv;
-      r = r - alpha * sv;
-      u = u - alpha * qv;
-      w = w - alpha * zv;
       m = precondition(w);
-      if (mine) ((taken & 1u) ? vec0 : vec1)[row] = pack(cvt<S>(m));
-      double* mine_part = halves[reductions & 1u];
+      if (mine) vec()[row] = publishedOf<S>(m);
+      double* const mine_part = partials();
       {
         double v[3] = {dot(r, u), dot(w, u), dot(r, r)};
         blockSum<3>(v);
@@ -550,10 +628,9 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
           for (int k = 0; k < 3; ++k) mine_part[k * G + part] = v[k];
       }
       if (!gangBarrier(arrive, G, s.sync, bar)) return;
-      // n = A m for the next iteration (m just published to vec[(taken + 1) & 1]), with the
-      // block partials requested first so that both round trips overlap
+      // n = A m for the next iteration, with the block partials requested first so that both round trips overlap
       if (stagedSums) requestBlockPartials(mine_part, partStage, 3u, G);
-      n = mine ? sellRow<S, U>(g, slice, lane, (taken & 1u) ? vec0 : vec1, tlCols, near, kept) : V3<double>{0, 0, 0};
+      n = product();
       double d[3];
       if (stagedSums) {
         cpAsyncWaitAll();
@@ -562,24 +639,20 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
       } else {
         sumBlocksAll<3>(mine_part, d, G);
       }
-      ++reductions;
       gammaNext = d[0];
       delta = d[1];
       length = d[2];
-      ++taken;
     }
     if (live) X[row] = pack(cvt<S>(x));
     if (part == 0 && threadIdx.x == 0) {
       const double residual = sqrt(length);
-      CgBodyDev c;
+      CgBodyDev c = s.cg[b];  // floor and start_res as written at the start
       c.squared = gamma;
       c.target = target;
-      c.floor = floor;
       c.length = length;
       c.stride = alpha;
       c.blend = beta;
-      c.start_res = startRes;
-      c.rel_res = residual / floor;
+      c.rel_res = residual / c.floor;
       c.taken = taken;
       c.done = 1u;
       c.pad0 = c.pad1 = 0;
@@ -587,7 +660,8 @@ __global__ void __launch_bounds__(TILE, 2) kPcgSell(Sys<S> s, SellDev<S> g, Gang
       CgReportDev rep = s.cgrep[b];
       rep.iterations += taken;
       rep.capped += (taken == st.limit && residual > target) ? 1u : 0u;
-      rep.applications += applications;
+      // r = right - A x, w = A u, and n = A m of every update but the last one the cap allows
+      rep.applications += (x0zero ? 1u : 2u) + taken - (taken != 0u && taken == st.limit ? 1u : 0u) + extra;
       rep.solves += 1u;
       rep.tangent_iterations += tangent ? taken : 0u;
       rep.worst_rel = fmax(rep.worst_rel, c.rel_res);
@@ -918,8 +992,8 @@ __global__ void __launch_bounds__(TILE, MINB)
     slotRows[j] = live ? (min(TILE, bd.node_end - tile * TILE) | (tile == bd.node_tile_begin ? 0x80000000u : 0u)) : 0u;
   }
   __syncthreads();
-  Vec4<S>* const vecA = g.vec;             // m of even phases (and of phase 0)
-  Vec4<S>* const vecB = g.vec + g.stride;  // u of the start, then m of odd phases
+  Published<S>* const vecA = g.vec;             // m of even phases (and of phase 0)
+  Published<S>* const vecB = g.vec + g.stride;  // u of the start, then m of odd phases
   // the FP64 recurrences, [8][Vp]: x, r, u, w, z, q, s, p (in an FP64 system x is X itself)
   constexpr bool wide = std::is_same_v<S, double>;
   Vec4<double>* const xd = wide ? reinterpret_cast<Vec4<double>*>(X) : state;
@@ -937,7 +1011,7 @@ __global__ void __launch_bounds__(TILE, MINB)
   const auto precondition = [&](uint32_t n, V3<double> v) {
     const Vec4<S> q0 = s.pre0[n], q1 = s.pre1[n];
     const Sym<double> P = {double(q0.x), double(q0.y), double(q0.z), double(q0.w), double(q1.x), double(q1.y)};
-    return roundTo<S>(symMul(P, v));
+    return roundPublished<S>(symMul(P, v));
   };
   // ---- start: r = right - A x (anchored rows 0), u = P r published; the recurrences start at 0
   for (uint32_t j = nextSlot(slotBody, 0u, slots); j < slots; j = nextSlot(slotBody, j + 1u, slots)) {
@@ -954,7 +1028,7 @@ __global__ void __launch_bounds__(TILE, MINB)
     const V3<double> uu = precondition(n, r);
     put(rd, n, r);
     put(u, n, uu);
-    vecB[n] = pack(cvt<S>(uu));
+    vecB[n] = publishedOf<S>(uu);
     if (x0zero) X[n] = zero4;
     if (!wide) xd[n] = x0zero ? zero4d : pack(cvt<double>(xyz(X[n])));
     zbuf[n] = zero4d;
@@ -974,7 +1048,7 @@ __global__ void __launch_bounds__(TILE, MINB)
         ww = sellRowOf<S, decltype(ld4cgOf(vecB)), U>(g, n >> 5, lane, ld4cgOf(vecB), static_cast<const uint32_t*>(nullptr));
       const V3<double> m = precondition(n, ww);
       put(w, n, ww);
-      vecA[n] = pack(cvt<S>(m));
+      vecA[n] = publishedOf<S>(m);
       const V3<double> r = get(rd, n), uu = get(u, n);
       const V3<double> rhs = cvt<double>(xyz(s.right[n]));
       sums[0] = dot(r, uu);
@@ -1018,8 +1092,8 @@ __global__ void __launch_bounds__(TILE, MINB)
     // the count of phase - 1's copy: retirements of this phase go to the other copy
     if (*(volatile int*)(((phase - 1u) & 1u) ? &s.sync->active_odd : &s.sync->active) <= 0) break;
     int* const retire = (phase & 1u) ? &s.sync->active_odd : &s.sync->active;
-    const Vec4<S>* const mcur = (phase & 1u) ? vecA : vecB;
-    Vec4<S>* const mnext = (phase & 1u) ? vecB : vecA;
+    const Published<S>* const mcur = (phase & 1u) ? vecA : vecB;
+    Published<S>* const mnext = (phase & 1u) ? vecB : vecA;
     uint32_t j = nextSlot(slotBody, 0u, slots);
     CgBodyDev cNow = {};
     if (j < slots) cNow = loadCg(&s.cg[slotBody[j]]);
@@ -1053,7 +1127,7 @@ __global__ void __launch_bounds__(TILE, MINB)
           if (!wide) X[n] = pack(cvt<S>(x));
           put(rd, n, r);
           if (full) {
-            const V3<double> m = cvt<double>(xyz(ld4cg(&mcur[n])));
+            const V3<double> m = wideOf(ld4cg(&mcur[n]));
             const V3<double> zz = nn + beta * get(zbuf, n);
             const V3<double> qq = m + beta * get(qbuf, n);
             const V3<double> u2 = uu - alpha * qq;
@@ -1062,7 +1136,7 @@ __global__ void __launch_bounds__(TILE, MINB)
             put(qbuf, n, qq);
             put(u, n, u2);
             put(w, n, w2);
-            mnext[n] = pack(cvt<S>(precondition(n, w2)));
+            mnext[n] = publishedOf<S>(precondition(n, w2));
             sums[0] = dot(r, u2);
             sums[1] = dot(w2, u2);
           }

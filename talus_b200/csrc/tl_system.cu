@@ -405,7 +405,7 @@ struct System final : SystemBase {
   uint32_t sellUpperCount = 0, sellColCache = 0;
   static constexpr uint32_t SELL_COL_CACHE_MAX = 32;  // column slots per thread in kPcgSell's shared memory
   DevBuf<S> sellVal;
-  DevBuf<Vec4<S>> sellVec;
+  DevBuf<Published<S>> sellVec;
   int pcg1PerSm[2][2] = {{0, 0}, {0, 0}};   // resident blocks per SM, [law][tangent]
   int batchPerSm[2][2] = {{0, 0}, {0, 0}};
   int pcg1DampPerSm[2] = {0, 0};             // corotated law with stiffness damping, [tangent]
