@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(CLUSTER_T, 1)
         CgReportDev rep = s.cgrep[0];
         rep.iterations += taken;
         rep.capped += (taken == st.limit && residual > target) ? 1u : 0u;
-        rep.applications += taken + (x0zero ? 0u : 1u);
+        rep.applications += taken + (x0zero ? 1u : 2u);  // A x, and A u of the start and of each update
         rep.solves += 1u;
         rep.tangent_iterations += tangent ? taken : 0u;
         rep.worst_rel = fmax(rep.worst_rel, o.rel_res);

@@ -152,3 +152,20 @@ def test_blocks_of_one_owner_take_the_same_decisions(cells, precision):
     for its, x in out[1:]:
         assert its == out[0][0]
         assert np.array_equal(x, out[0][1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells", [(1, 1, 7), (8, 7, 7), (15, 16, 15)])
+def test_operator_applications_are_those_of_the_elementwise_form(cells):
+    """The same order and in FP64 the same iterations, so the same products with the operator."""
+    mesh = tb.box_mesh(cells, voxel=0.1, jitter=0.01, seed=3)
+    mat = tb.PhysicalMaterial(density=1000.0, youngs_modulus=1e6, poissons_ratio=0.3)
+    out = {}
+    for form in ("auto", "elementwise"):
+        s = tb.System(mesh, [mat], tb.FP64)
+        s.set_solver(form)
+        s.set_state(tb.rest_state(mesh))
+        reports = [s.step(tb.Settings(cg_iterations=1000), GRAVITY, DT)[0] for _ in range(3)]
+        out[form] = [(r.cg_iterations, r.operator_applications) for r in reports]
+        s.close()
+    assert out["auto"] == out["elementwise"]
