@@ -1544,7 +1544,7 @@ struct System final : SystemBase {
 
   // ---------------------------------------------------------- launches ----
 
-  void check() {
+  void check() {  // after each launch by <<<>>>, which it counts
     TL_CUDA(cudaGetLastError());
     ++launches;
   }
@@ -1626,7 +1626,6 @@ struct System final : SystemBase {
       if (profiling) mark(1, true);  // the operator assembly counts as assembly time
       assembleSell(s, g, blocks, idx, damp, tangent, ps);
       check();
-      ++launches;
       if (profiling) {
         mark(1, false);
         mark(2, true);
@@ -1648,7 +1647,6 @@ struct System final : SystemBase {
       if (profiling) mark(1, true);
       assembleSell(s, g, blocks, idx, damp, tangent, ps);
       check();
-      ++launches;
       if (profiling) {
         mark(1, false);
         mark(2, true);
@@ -1988,7 +1986,6 @@ struct System final : SystemBase {
     if (profiling) mark(1, true);
     assembleSell(s, g, blocks, law == TL_LAW_SNH ? 1 : 0, hasDamping && law != TL_LAW_SNH, tangent, pass);
     check();
-    ++launches;
     if (profiling) {
       mark(1, false);
       mark(2, true);
@@ -2143,7 +2140,6 @@ struct System final : SystemBase {
     }
     kInversionCheck<S><<<elemTiles, TILE, 0, st>>>(view());
     check();
-    ++launches;
     BodyAccDev* ha = hAcc.get(B);
     acc.download(ha, B, st);
     TL_CUDA(cudaStreamSynchronize(st));
@@ -2347,6 +2343,7 @@ struct System final : SystemBase {
       if (yieldsLaw) element(law, u.ptr, nullptr, pass, EM_MAPPING | EM_COMMIT, 0.0);
     }
     kStepEnd<S><<<nodeTiles, TILE, 0, st>>>(view());
+    check();
     finalize(0);
     finalize(2);
     acc.download(hAcc.ptr, B, st);

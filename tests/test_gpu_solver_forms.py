@@ -177,3 +177,31 @@ def test_launch_shape_values_are_checked():
             tb._capi.check(tb._capi.lib().tl_system_tune_shape(s.handle, knob, value), s.context.handle)
         assert e.value.status == tb._capi.TL_ERR_ARG
     s.close()
+
+
+def test_each_launch_is_counted_once():
+    """A solve in a cluster is two launches, the operator's assembly and the PCG; over the whole grid a third one
+    resets the barrier's words; element by element there is no assembly.  A batch's step counts the same replayed from
+    its graph, but for the opening's: the inversion test alone, or with it the accumulators' reset and the substep
+    choice before and after."""
+    mesh, mat = elastic_block()
+    per = {}
+    for form in ("auto", "assembled-two-phase", "elementwise"):
+        s = tb.System(mesh, [mat], tb.FP64)
+        s.set_solver(form)
+        s.set_state(tb.rest_state(mesh))
+        r = s.step(tb.Settings(), GRAVITY, DT)[0]
+        per[form] = r.kernel_launches
+        solves = r.cg_solves
+        s.close()
+    assert per["assembled-two-phase"] - per["auto"] == solves
+    assert per["auto"] == per["elementwise"]
+    out = []
+    for graph in (False, True):
+        s = tb.System([mesh, mesh], [[mat], [mat]], tb.FP64)
+        s.tune(graph=graph)
+        for b in range(2):
+            s.set_state(tb.rest_state(mesh), b)
+        out.append(s.step(tb.Settings(), GRAVITY, DT)[0].kernel_launches)
+        s.close()
+    assert out[1] - out[0] == 3
