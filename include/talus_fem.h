@@ -202,9 +202,11 @@ int32_t tl_system_tune_shape(tl_system* system, uint32_t knob, uint32_t value);
  * the 3x3 node blocks once per solve and iterates on that matrix (about 40
  * bytes per nonzero block in FP32, 76 in FP64);
  * TL_SOLVER_ELEMENTWISE always iterates element by element;
- * TL_SOLVER_AUTO (default) is ASSEMBLED.  A single body of up to 5,120 nodes
- * then solves inside one thread-block cluster (kPcgCluster) where its rows
- * fit the cluster's shared memory, others over the whole GPU (kPcgSell).
+ * TL_SOLVER_AUTO (default) is ASSEMBLED, but for a single body of more nodes
+ * than the resident grid has threads (75,776 on a B200), which it iterates
+ * element by element.  A single body of up to 5,120 nodes solves inside one
+ * thread-block cluster (kPcgCluster) where its rows fit the cluster's shared
+ * memory, others over the whole GPU (kPcgSell).
  * Both forms apply the same operator; they differ in rounding.  On the
  * assembled matrix ASSEMBLED and AUTO iterate each body of a batch with its
  * own group of blocks, in the pipelined order with one barrier per iteration
@@ -212,9 +214,11 @@ int32_t tl_system_tune_shape(tl_system* system, uint32_t knob, uint32_t value);
  * the same iterates in exact arithmetic, step every body of the system in
  * lockstep: TL_SOLVER_ASSEMBLED_TWO_PHASE, the textbook order with two grid
  * barriers per iteration, and TL_SOLVER_ASSEMBLED_PIPELINED, the pipelined
- * order with its recurrences in memory (eight FP64 vectors per node).  A
- * system with a body of more nodes than the resident grid has threads takes
- * the pipelined one in FP64 and the two-phase one in FP32-mixed. */
+ * order with its recurrences in memory (eight FP64 vectors per node).  They
+ * apply to batches, and to single bodies too large for kPcgSell; a smaller
+ * single body runs kPcgSell in both.  A system with a body of more nodes than
+ * the resident grid has threads takes the pipelined one in FP64 and the
+ * two-phase one in FP32-mixed (a single such body in ASSEMBLED). */
 #define TL_SOLVER_AUTO 0u
 #define TL_SOLVER_ASSEMBLED 1u
 #define TL_SOLVER_ELEMENTWISE 2u

@@ -1121,10 +1121,17 @@ struct System final : SystemBase {
     g.vec = sellVec.ptr;
     return g;
   }
-  // Whether this system's PCG runs on the assembled matrix, which TL_SOLVER_AUTO always chooses: with one block per
-  // SM kPcgSell overtakes the element-by-element kernel for every body past a cluster's (5,202 nodes, a frame: 1.19
+  // Whether this system's PCG may run on the assembled matrix, which TL_SOLVER_AUTO chooses wherever kPcgCluster or
+  // kPcgSell takes the bodies: with one block per SM kPcgSell overtakes the element-by-element kernel for every body past a cluster's (5,202 nodes, a frame: 1.19
   // against 1.38 ms in FP32-mixed, 1.40 against 1.59 in FP64, the assembly included).
   bool assembledForm() const { return sellReady && solverForm != TL_SOLVER_ELEMENTWISE; }
+  // Whether a solve that kPcgSell does not take runs in one of the lockstep orders.  A single body of more rows than the
+  // resident grid has threads keeps the element-by-element route in TL_SOLVER_AUTO.  ASSEMBLED asks for the lockstep one
+  // (two steps at the default settings, 91,908 nodes: FP64 17.4 ms element by element, 15.5 assembled, FP32-mixed 9.5
+  // and 10.3; 545,025 nodes: 94.9 and 70.9, 55.8 and 46.7).
+  bool lockstepForm() const {
+    return assembledForm() && batchSellPerSm > 0 && (B > 1 || solverForm != TL_SOLVER_AUTO);
+  }
   // Grid of kPcgSell, or 0 where it does not run: a body with more rows than the grid has threads, or a batch in one
   // of the lockstep orders.
   int sellGrid() const {
@@ -1632,7 +1639,7 @@ struct System final : SystemBase {
       }
       void* args[] = {&s, &g, &gang, &X, &ps, &xz, &tg};
       TL_CUDA(cudaLaunchCooperativeKernel(sellKernel(), dim3(sellG), dim3(TILE), args, sellColBytes(), st));
-    } else if (B == 1) {  // single body, element by element: two-level assembly, per-block partials
+    } else if (B == 1 && !lockstepForm()) {  // single body, element by element: two-level assembly, per-block partials
       if (profiling) mark(2, true);
       void* args[] = {&s, &X, &xz};
       const void* fn = idx ? (tangent ? (const void*)kPcg1<S, 1, true> : (const void*)kPcg1<S, 1, false>)
@@ -1641,7 +1648,7 @@ struct System final : SystemBase {
       const int perSm = damp ? pcg1DampPerSm[tangent ? 1 : 0] : pcg1PerSm[idx][tangent ? 1 : 0];
       TL_CUDA(cudaLaunchCooperativeKernel(fn, dim3(gridOf(perSm)), dim3(TILE), args,
                                           sizeof(TileCache), st));
-    } else if (assembledForm() && batchSellPerSm > 0) {  // batch, or a body too large for kPcgSell
+    } else if (lockstepForm()) {  // a lockstep order, or a body too large for kPcgSell
       SellDev<S> g = sellView();
       const unsigned blocks = (sellUpperCount + TILE - 1) / TILE;
       if (profiling) mark(1, true);
@@ -1652,8 +1659,9 @@ struct System final : SystemBase {
         mark(2, true);
       }
       Vec4<S>* p2 = sellP2.ptr;
-      // the batch's order: measured on 512 uneven bodies solved to 1e-6, the pipelined
-      // order (FP64 recurrences) is the faster in FP64 and the two-phase one in FP32-mixed
+      // the faster order of each precision: two steps of a 91,908-node body and 20 of 1,000 nodes, pipelined against
+      // two-phase, FP64 19.0 and 19.3 ms at the default settings, 47.4 and 49.7 to 1e-6; FP32-mixed 13.1 and 11.0,
+      // 31.4 and 27.6
       const bool twoPhase = solverForm == TL_SOLVER_ASSEMBLED_TWO_PHASE ||
                             (solverForm != TL_SOLVER_ASSEMBLED_PIPELINED && sizeof(S) == 4);
       int perSm = twoPhase ? batchSellPerSm : batchPipePerSm;

@@ -205,3 +205,18 @@ def test_each_launch_is_counted_once():
         out.append(s.step(tb.Settings(), GRAVITY, DT)[0].kernel_launches)
         s.close()
     assert out[1] - out[0] == 3
+
+
+@pytest.mark.parametrize("form", ["assembled", "assembled-two-phase", "assembled-pipelined"])
+@pytest.mark.parametrize("precision,tol", [(tb.FP64, 1e-10), (tb.FP32_MIXED, 1e-5)])
+def test_assembled_forms_of_a_body_too_large_for_one_row_per_thread(form, precision, tol):
+    """The assembled operator is what runs there: each solve launches its assembly, which the element-by-element form
+    has not."""
+    mesh = tb.box_mesh((68, 36, 35), voxel=0.1)
+    mat = tb.PhysicalMaterial(density=1000.0, youngs_modulus=1e6, poissons_ratio=0.3)
+    xa, ra = run(form, precision, mesh, mat, tb.Settings(), 2)
+    xe, re = run("elementwise", precision, mesh, mat, tb.Settings(), 2)
+    assert relative_error(xa, xe, mesh.rest_positions) <= tol
+    assert [r["kernel_launches"] - r["cg_solves"] for r in ra] == [r["kernel_launches"] for r in re]
+    if precision == tb.FP64:
+        assert [r["cg_iterations"] for r in ra] == [r["cg_iterations"] for r in re]
