@@ -1658,7 +1658,8 @@ __device__ __forceinline__ CgBodyDev loadCg(const CgBodyDev* p) {
   c.rel_res = __ldcg(&p->rel_res);
   c.taken = __ldcg(&p->taken);
   c.done = __ldcg(&p->done);
-  c.pad0 = c.pad1 = 0;
+  c.pad0 = __ldcg(&p->pad0);
+  c.pad1 = __ldcg(&p->pad1);
   return c;
 }
 
