@@ -947,18 +947,39 @@ __global__ void __launch_bounds__(TILE, MINB)
 // two copies: phase k reads copy k & 1 and retires bodies from that copy
 // only; a body retired in phase k leaves copy (k + 1) & 1 in phase k + 1,
 // through the block that holds its first tile.
-constexpr uint32_t PIPE_FULL = 0u;  // kinds of a body's next update
-constexpr uint32_t PIPE_LAST = 1u;
+//
+// A body's recurrences are replaced as kPcgSell's are, over the phases
+// PIPE_OPEN to PIPE_Q, each of which multiplies what the phase before it
+// published and publishes the next vector: x (FP64), p, P r, P s, and m at last.
+constexpr uint32_t PIPE_FULL = 0u;  // kinds of a body's next phase: an update,
+constexpr uint32_t PIPE_LAST = 1u;  // the last one the cap allows,
+constexpr uint32_t PIPE_OPEN = 2u;  // or a step of the replacement
+constexpr uint32_t PIPE_X = 3u;     // r = right - A x
+constexpr uint32_t PIPE_P = 4u;     // s = A p
+constexpr uint32_t PIPE_U = 5u;     // w = A u
+constexpr uint32_t PIPE_Q = 6u;     // z = A q
 
 // kPcgSell's loop top for one body (thread 0 of its last tile): given the
 // sums gamma' = r.u, delta = w.u and |r|^2 of the current iterate, either stop
-// or set alpha, beta and the kind of the next update.
+// or set alpha, beta and the kind of the next phase.  rel_res, which is not
+// known before the solve ends, holds the upper words of the largest r.u and r.r
+// since the last replacement, 0 after one.
+template <class S>
 __device__ __forceinline__ void pipeDecide(CgBodyDev& c, double gammaNext, double delta, uint32_t limit,
                                            uint32_t phase) {
   if (c.taken >= limit || sqrt(c.length) <= c.target) {
     c.done = phase + 1u;
     return;
   }
+  const int length = __double2hiint(c.length), gamma = __double2hiint(gammaNext);
+  const int mostLength = __double2hiint(c.rel_res), mostGamma = __double2loint(c.rel_res);
+  if (mostLength != 0 && (length < mostLength - SELL_FALL || gamma < mostGamma - SELL_FALL)) {
+    c.rel_res = 0.0;
+    c.pad0 = PIPE_OPEN;
+    c.pad1 += sizeof(S) == 8 ? 4u : 3u;
+    return;
+  }
+  c.rel_res = __hiloint2double(max(mostLength, length), max(mostGamma, gamma));
   const double b = c.taken ? gammaNext / c.squared : 0.0;
   const double curvature = c.taken ? delta - b * gammaNext / c.stride : delta;  // p.A p
   if (!(curvature > 0.0) || !(gammaNext > 0.0)) {
@@ -970,6 +991,63 @@ __device__ __forceinline__ void pipeDecide(CgBodyDev& c, double gammaNext, doubl
   c.squared = gammaNext;
   c.pad0 = c.taken + 1u >= limit ? PIPE_LAST : PIPE_FULL;
   if (c.pad0 == PIPE_FULL) c.pad1 += 1u;  // the matvec n = A m of the update
+}
+
+// A replacement's phase for row n; r.u, w.u and r.r in the last one.  Out of
+// line, as its registers would cost the update's (two FP64 steps of a body of
+// 91,908 nodes and 20 small ones: 20.6 ms inline, 19.6 so, 19.0 without it).
+template <class S> struct PipeRow {
+  const uint8_t* anch;
+  const Vec4<S>*right, *pre0, *pre1;
+  Vec4<S>* X;
+  Vec4<double>* state;
+  const Published<S>* mcur;
+  Published<S>* mnext;
+  uint32_t Vp;
+};
+template <class S, uint32_t U>
+static __device__ __noinline__ V3<double> pipeReplace(PipeRow<S> at, const uint32_t* sliceStart, const uint32_t* col,
+                                                      S* val, uint32_t n, uint32_t kind) {
+  constexpr bool wide = std::is_same_v<S, double>;
+  const auto plane = [&](uint32_t k) { return &at.state[k * size_t(at.Vp) + n]; };
+  Vec4<double> *const r = plane(1), *const u = plane(2), *const w = plane(3), *const z = plane(4), *const q = plane(5),
+               *const sv = plane(6), *const p = plane(7);
+  const auto precondition = [&](V3<double> v) {
+    const Vec4<S> q0 = at.pre0[n], q1 = at.pre1[n];
+    const Sym<double> P = {double(q0.x), double(q0.y), double(q0.z), double(q0.w), double(q1.x), double(q1.y)};
+    return roundPublished<S>(symMul(P, v));
+  };
+  V3<double> y = {0, 0, 0}, v = {0, 0, 0}, sums = {0, 0, 0};
+  if (kind != PIPE_OPEN && !at.anch[n]) {
+    SellDev<S> g;
+    g.slice_start = sliceStart;
+    g.col = col;
+    g.val = val;
+    g.col_cache = 0;
+    y = sellRowOf<S, decltype(ld4cgOf(at.mcur)), U>(g, n >> 5, threadIdx.x & 31u, ld4cgOf(at.mcur),
+                                                    static_cast<const uint32_t*>(nullptr));
+  }
+  if (wide && kind == PIPE_OPEN) {
+    v = cvt<double>(xyz(at.X[n]));
+  } else if (kind <= PIPE_X) {
+    if (kind == PIPE_X) *r = pack(at.anch[n] ? V3<double>{0, 0, 0} : cvt<double>(xyz(at.right[n])) - y);
+    v = roundPublished<S>(xyz(*p));
+    *p = pack(v);
+  } else if (kind == PIPE_P) {
+    *sv = pack(y);
+    v = precondition(xyz(*r));
+    *u = pack(v);
+  } else if (kind == PIPE_U) {
+    *w = pack(y);
+    v = precondition(xyz(*sv));
+    *q = pack(v);
+  } else {
+    *z = pack(y);
+    v = precondition(xyz(*w));
+    sums = {dot(xyz(*r), xyz(*u)), dot(xyz(*w), xyz(*u)), dot(xyz(*r), xyz(*r))};
+  }
+  at.mnext[n] = publishedOf<S>(v);
+  return sums;
 }
 
 template <class S, uint32_t U = BATCH_ROW_GROUP, int MINB = BATCH_BLOCKS>
@@ -1072,7 +1150,7 @@ __global__ void __launch_bounds__(TILE, MINB)
         c.target = s.step[b].tolerance * c.floor;
         c.length = tot[2];
         c.start_res = sqrt(tot[2]) / c.floor;
-        c.rel_res = c.start_res;
+        c.rel_res = 0.0;
         c.squared = 0.0;
         c.stride = 0.0;
         c.blend = 0.0;
@@ -1080,7 +1158,7 @@ __global__ void __launch_bounds__(TILE, MINB)
         c.done = 0;
         c.pad0 = PIPE_FULL;
         c.pad1 = (x0zero ? 0u : 1u) + 1u;  // r = right - A x and w = A u
-        pipeDecide(c, tot[0], tot[1], s.step[b].limit, 0u);
+        pipeDecide<S>(c, tot[0], tot[1], s.step[b].limit, 0u);
         s.cg[b] = c;
         __threadfence();
         if (c.done) atomicSub(&s.sync->active, 1);
@@ -1109,8 +1187,17 @@ __global__ void __launch_bounds__(TILE, MINB)
         const uint32_t n = tile * TILE + threadIdx.x;
         const double alpha = cNow.stride, beta = cNow.blend;
         double sums[3] = {0.0, 0.0, 0.0};
-        if (threadIdx.x < (rowsWord & 0x7fffffffu)) {
-          const bool full = cNow.pad0 == PIPE_FULL;
+        const uint32_t kind = cNow.pad0;
+        if (kind >= PIPE_OPEN) {
+          if (threadIdx.x < (rowsWord & 0x7fffffffu)) {
+            const PipeRow<S> at = {s.anch, s.right, s.pre0, s.pre1, X, state, mcur, mnext, s.Vp};
+            const V3<double> t = pipeReplace<S, U>(at, g.slice_start, g.col, g.val, n, kind);
+            sums[0] = t.x;
+            sums[1] = t.y;
+            sums[2] = t.z;
+          }
+        } else if (threadIdx.x < (rowsWord & 0x7fffffffu)) {
+          const bool full = kind == PIPE_FULL;
           // the matvec first: its round trips are the phase's latency
           V3<double> nn = {0, 0, 0};
           if (full && !s.anch[n])
@@ -1153,12 +1240,16 @@ __global__ void __launch_bounds__(TILE, MINB)
           sumTiles<3>(s.part, bd.node_tile_begin, bd.node_tile_end, tot);
           if (threadIdx.x == 0) {
             CgBodyDev c = loadCg(&s.cg[b]);
-            c.length = tot[2];
-            c.taken += 1u;
-            if (c.pad0 == PIPE_LAST)
-              c.done = phase + 1u;
-            else
-              pipeDecide(c, tot[0], tot[1], s.step[b].limit, phase);
+            if (c.pad0 >= PIPE_OPEN && c.pad0 < PIPE_Q) {
+              c.pad0 = !wide && c.pad0 == PIPE_OPEN ? PIPE_P : c.pad0 + 1u;
+            } else {
+              c.length = tot[2];
+              if (c.pad0 < PIPE_OPEN) c.taken += 1u;
+              if (c.pad0 == PIPE_LAST)
+                c.done = phase + 1u;
+              else
+                pipeDecide<S>(c, tot[0], tot[1], s.step[b].limit, phase);
+            }
             s.cg[b] = c;
             __threadfence();
             if (c.done) atomicSub(retire, 1);

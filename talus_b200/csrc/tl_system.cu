@@ -1127,8 +1127,8 @@ struct System final : SystemBase {
   bool assembledForm() const { return sellReady && solverForm != TL_SOLVER_ELEMENTWISE; }
   // Whether a solve that kPcgSell does not take runs in one of the lockstep orders.  A single body of more rows than the
   // resident grid has threads keeps the element-by-element route in TL_SOLVER_AUTO.  ASSEMBLED asks for the lockstep one
-  // (two steps at the default settings, 91,908 nodes: FP64 17.4 ms element by element, 15.5 assembled, FP32-mixed 9.5
-  // and 10.3; 545,025 nodes: 94.9 and 70.9, 55.8 and 46.7).
+  // (two steps at the default settings, 91,908 nodes: FP64 17.4 ms element by element, 16.1 assembled, FP32-mixed 9.5
+  // and 10.2; 545,025 nodes: 94 and 73, 55 and 46).
   bool lockstepForm() const {
     return assembledForm() && batchSellPerSm > 0 && (B > 1 || solverForm != TL_SOLVER_AUTO);
   }
@@ -1659,9 +1659,9 @@ struct System final : SystemBase {
         mark(2, true);
       }
       Vec4<S>* p2 = sellP2.ptr;
-      // the faster order of each precision: two steps of a 91,908-node body and 20 of 1,000 nodes, pipelined against
-      // two-phase, FP64 19.0 and 19.3 ms at the default settings, 47.4 and 49.7 to 1e-6; FP32-mixed 13.1 and 11.0,
-      // 31.4 and 27.6
+      // FP32-mixed: the faster order (two steps of a 91,908-node body and 20 of 1,000 nodes, two-phase against pipelined:
+      // 10.6 and 13.2 ms at the default settings, 26.5 and 32.5 to 1e-6).  FP64: the two are within 2% there (19.4 and
+      // 19.6, 49.5 and 50.5), and the pipelined order is 8% faster for such a body alone (17.5 and 16.1)
       const bool twoPhase = solverForm == TL_SOLVER_ASSEMBLED_TWO_PHASE ||
                             (solverForm != TL_SOLVER_ASSEMBLED_PIPELINED && sizeof(S) == 4);
       int perSm = twoPhase ? batchSellPerSm : batchPipePerSm;

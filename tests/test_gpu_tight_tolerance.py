@@ -70,3 +70,13 @@ def test_layered_body(precision, tolerance):
     top = mesh.rest_positions[mesh.tet_nodes.astype(np.int64)][:, :, 1].mean(1) > 0.85
     reports = stepped(mesh, [material(1e5, 0.3)], precision, tolerance, "auto", youngs=np.where(top, 1e9, 1e5))
     check(reports, tolerance)
+
+
+@pytest.mark.parametrize("precision,tolerance", [(tb.FP32_MIXED, 1e-5), (tb.FP32_MIXED, 1e-6), (tb.FP64, 1e-8),
+                                                 (tb.FP64, 1e-12)])
+def test_lockstep_pipelined_batch(precision, tolerance):
+    """The lockstep pipelined order: bodies replace their recurrences in different phases, beside others that update,
+    stop early or fill less than a tile."""
+    meshes = [tb.box_mesh(c, voxel=0.1) for c in ((12, 11, 10), (3, 30, 4), (2, 2, 2), (9, 20, 9), (7, 7, 3))]
+    mats = [[material(e, 0.35)] for e in (1e8, 3e7, 1e5, 1e8, 1e6)]
+    check(stepped(meshes, mats, precision, tolerance, "assembled-pipelined"), tolerance)
