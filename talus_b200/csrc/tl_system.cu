@@ -1737,6 +1737,7 @@ struct System final : SystemBase {
   // and half of the memory that is free, are what a solver state may take of the device's memory.
   static constexpr uint64_t INVERSE_MAX = uint64_t(24) << 30;
   bool fInverse = false, fLean = false;
+  bool dfReady = false;  // the ordering, in the form that is to run, is on the device
   uint32_t fLongRows = 0, fShortRows = 0, fGroups = 0, fChunks = 0;
   DevBuf<double> dfX, dfB, dfYs;
   DevBuf<uint64_t> dfOff;
@@ -1763,13 +1764,14 @@ struct System final : SystemBase {
   void useFactor(uint32_t enable, uint32_t budget) override {
     if (!enable) {
       factorOn = false;
+      dropFactor();
       return;
     }
     if (B != 1) throw StatusError{TL_ERR_UNSUPPORTED, "a solver state is held for one-body systems"};
     if (!sellReady) throw StatusError{TL_ERR_UNSUPPORTED, "the factored PCG needs the assembled operator"};
     if (hencky) throw StatusError{TL_ERR_UNSUPPORTED, "the factor is made for the small-strain path"};
     factorOn = true;
-    if (fLean != (enable == TL_FACTOR_LEAN)) fHost.analyzed = false;
+    if (fLean != (enable == TL_FACTOR_LEAN)) dropFactor();
     fLean = enable == TL_FACTOR_LEAN;
     factorBudget = budget;
     fHost.ready = false;
@@ -1781,6 +1783,20 @@ struct System final : SystemBase {
       if (factorPerSm < 1 || inversePerSm < 1)
         throw StatusError{TL_ERR_UNSUPPORTED, "the factored PCG grid cannot be resident"};
     }
+  }
+  // Gives the device's part of the state back; the host's ordering stays, a factor is made and sent again.
+  void dropFactor() {
+    TL_CUDA(cudaStreamSynchronize(st));
+    dfReady = false;
+    for (DevBuf<uint32_t>* b : {&dfPerm, &dfIperm, &dfRowStart, &dfRowCol, &dfColStart, &dfColRow, &dfFlags, &dfTicket,
+                                &dfSnStart, &dfRowSplit, &dfColSplit, &dfFirst, &dfRows, &dfAnc})
+      b->alloc(0);
+    for (DevBuf<int32_t>* b : {&dfSnChild, &dfSnParent}) b->alloc(0);
+    for (DevBuf<double>* b : {&dfRowBlk, &dfColBlk, &dfDiagInv, &dfFrame, &dfPart, &dfX, &dfB, &dfYs}) b->alloc(0);
+    for (DevBuf<Vec4<double>>* b : {&dfY, &dfW, &dfRef, &dfRhs}) b->alloc(0);
+    for (DevBuf<Vec4<S>>* b : {&dfR, &dfD, &dfD2, &dfQ, &dfZ, &dfRestart}) b->alloc(0);
+    for (DevBuf<uint4>* b : {&dfGroup, &dfChunk}) b->alloc(0);
+    dfOff.alloc(0);
   }
   void factorStats(tl_factor_stats* out) override {
     *out = fStats;
@@ -1838,6 +1854,9 @@ struct System final : SystemBase {
     getNodes(bd, h, u, x.data(), true);
     if (!fHost.analyzed || fHost.nodes != V) {  // analyzeSystem (factor.cc:549-565), once per mesh
       fHost.analyze(V, fAnch.data(), fTets, h.rest.data());
+      dfReady = false;
+    }
+    if (!dfReady) {
       auto put = [&](DevBuf<uint32_t>& d, const std::vector<uint32_t>& v) {
         d.alloc(std::max<size_t>(v.size(), 1));
         d.upload(v.data(), v.size(), st);
@@ -1908,6 +1927,7 @@ struct System final : SystemBase {
         b->alloc(Vp);
         b->zero(st);
       }
+      dfReady = true;
     }
     std::vector<double> blocks(size_t(144) * T), diag(size_t(9) * V, 0.0);
     parallelFor(T, [&](size_t e0, size_t e1) {

@@ -55,3 +55,32 @@ def test_form_can_change_between_steps():
         capi.check(capi.lib().tl_system_use_factor(s.handle, enable, 32), s.context.handle)
         assert s.step(tb.Settings(), GRAVITY, DT)[0].non_finite == 0
     s.close()
+
+
+@pytest.mark.parametrize("enable", [1, 2])
+def test_a_dropped_state_gives_its_memory_back(enable):
+    """16 x 8 x 8 cells: 17 MB of inverse, or 12 MB of factor blocks.  Allocations come in pieces of 2 MB."""
+    torch = pytest.importorskip("torch")
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    mesh, mat = plastic_block((16, 8, 8))
+    s = tb.System(mesh, [mat], tb.FP64)
+    s.set_state(tb.rest_state(mesh))
+    use = lambda e: capi.check(capi.lib().tl_system_use_factor(s.handle, e, 32), s.context.handle)  # noqa: E731
+    use(enable)  # the kernels' own memory, once
+    s.step(tb.Settings(), GRAVITY, DT)
+    use(0)
+    s.step(tb.Settings(), GRAVITY, DT)
+    before = free()
+    use(enable)
+    first = s.step(tb.Settings(), GRAVITY, DT)[0].cg_iterations
+    assert free() < before - (8 << 20)
+    use(0)
+    assert free() >= before - (2 << 20)
+    assert s.step(tb.Settings(), GRAVITY, DT)[0].non_finite == 0
+    use(enable)
+    assert s.step(tb.Settings(), GRAVITY, DT)[0].cg_iterations > 0 and first > 0
+    s.close()
