@@ -247,7 +247,10 @@ int32_t tl_system_set_solver(tl_system* system, uint32_t form);
  * half of the free device memory;
  * enable = TL_FACTOR_LEAN solves with the factor itself (kPcgFactor), which
  * takes a fifth of the memory or less and 14 times as long or more.  Both
- * apply the same factor; they differ in rounding. */
+ * apply the same factor; they differ in rounding.  tl_factor_stats::form says
+ * which one runs: it is chosen when the first factor after enabling is made,
+ * by the device memory that is free then.  enable = 0 gives the memory back. */
+#define TL_FACTOR_INVERSE 1u
 #define TL_FACTOR_LEAN 2u
 int32_t tl_system_use_factor(tl_system* system, uint32_t enable, uint32_t factor_budget);
 
@@ -277,7 +280,7 @@ typedef struct tl_factor_stats {
   uint32_t spent_after_refresh;
   uint32_t refreshed_at_age;
   uint32_t factor_applications;
-  uint32_t reserved;
+  uint32_t form;  /* how the factor is applied: 0 none made yet, TL_FACTOR_INVERSE, TL_FACTOR_LEAN */
   uint64_t factor_nonzeros;
   double refactor_seconds;  /* host time spent making the factor */
 } tl_factor_stats;

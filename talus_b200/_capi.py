@@ -38,6 +38,8 @@ TL_SOLVER_ASSEMBLED = 1
 TL_SOLVER_ELEMENTWISE = 2
 TL_SOLVER_ASSEMBLED_TWO_PHASE = 3
 TL_SOLVER_ASSEMBLED_PIPELINED = 4
+TL_FACTOR_INVERSE = 1
+TL_FACTOR_LEAN = 2
 TL_SHAPE_ROW_GROUP = 0
 TL_SHAPE_BATCH_BLOCKS = 1
 TL_PLASTICITY_SMALL_STRAIN = 0
@@ -132,11 +134,11 @@ class tl_factor_stats(C.Structure):
                 ("system_nonzeros", C.c_uint64), ("generation", C.c_uint64)] + \
                [(n, C.c_uint32) for n in ("refresh_requests", "refactors", "retries", "retries_failed",
                                           "wasted_iterations", "spent_before_refresh", "spent_after_refresh",
-                                          "refreshed_at_age", "factor_applications", "reserved")] + \
+                                          "refreshed_at_age", "factor_applications", "form")] + \
                [("factor_nonzeros", C.c_uint64), ("refactor_seconds", C.c_double)]
 
     def as_dict(self) -> dict:
-        return {name: getattr(self, name) for name, _ in self._fields_ if name != "reserved"}
+        return {name: getattr(self, name) for name, _ in self._fields_ if name != "form"}
 
 
 class tl_rollout_desc(C.Structure):

@@ -1805,6 +1805,7 @@ struct System final : SystemBase {
     out->ready = fHost.ready ? 1u : 0u;
     out->system_nonzeros = fHost.systemNonZeros;
     out->factor_nonzeros = fHost.factorNonZeros();
+    out->form = !dfReady ? 0u : fInverse ? TL_FACTOR_INVERSE : TL_FACTOR_LEAN;
   }
   FactorDev factorView() {
     FactorDev f;

@@ -292,6 +292,13 @@ class System:
         check(capi.lib().tl_system_factor_stats(self.handle, C.byref(out)), self.context.handle)
         return out.as_dict()
 
+    def factor_form(self):
+        """How the solver state's factor is applied (tl_factor_stats::form):
+        "inverse", "lean", or None before one is made."""
+        out = capi.tl_factor_stats()
+        check(capi.lib().tl_system_factor_stats(self.handle, C.byref(out)), self.context.handle)
+        return {capi.TL_FACTOR_INVERSE: "inverse", capi.TL_FACTOR_LEAN: "lean"}.get(out.form)
+
     def set_solver(self, form: str = "auto"):
         """PCG operator form of a system (tl_system_set_solver): "auto",
         "assembled" (3x3 node blocks assembled once per solve),

@@ -84,3 +84,17 @@ def test_a_dropped_state_gives_its_memory_back(enable):
     use(enable)
     assert s.step(tb.Settings(), GRAVITY, DT)[0].cg_iterations > 0 and first > 0
     s.close()
+
+
+def test_the_form_that_runs_is_reported():
+    mesh, mat = plastic_block((4, 3, 4))
+    s = tb.System(mesh, [mat], tb.FP64)
+    s.set_state(tb.rest_state(mesh))
+    assert s.factor_form() is None
+    for enable, form in ((1, "inverse"), (2, "lean"), (1, "inverse")):
+        capi.check(capi.lib().tl_system_use_factor(s.handle, enable, 32), s.context.handle)
+        s.step(tb.Settings(), GRAVITY, DT)
+        assert s.factor_form() == form
+    capi.check(capi.lib().tl_system_use_factor(s.handle, 0, 32), s.context.handle)
+    assert s.factor_form() is None
+    s.close()
