@@ -203,8 +203,9 @@ int32_t tl_system_tune_shape(tl_system* system, uint32_t knob, uint32_t value);
  * bytes per nonzero block in FP32, 76 in FP64);
  * TL_SOLVER_ELEMENTWISE always iterates element by element;
  * TL_SOLVER_AUTO (default) is ASSEMBLED, but for a single body of more nodes
- * than the resident grid has threads (75,776 on a B200), which it iterates
- * element by element.  A single body of up to 5,120 nodes solves inside one
+ * than the resident grid has threads (75,776 on a B200) or with a node of many
+ * neighbours (over 31, up to 127 in a small body), which it iterates element
+ * by element.  A single body of up to 5,120 nodes solves inside one
  * thread-block cluster (kPcgCluster) where its rows fit the cluster's shared
  * memory, others over the whole GPU (kPcgSell).
  * Both forms apply the same operator; they differ in rounding.  On the

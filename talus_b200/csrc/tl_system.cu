@@ -996,7 +996,16 @@ struct System final : SystemBase {
     TL_CUDA(cudaStreamSynchronize(st));
     sellReady = sellPerSm > 0 || batchSellPerSm > 0;
     buildCluster(h);
+    sellHub = B == 1 && (cluster.kernel ? (widest + cluster.dev.parts - 1) / cluster.dev.parts : widest) > HUB_SLOTS;
   }
+  // A row's column slots are one thread's chain in kPcgSell, and shared by a slice's workers in kPcgCluster, so one node
+  // with many neighbours sets the time of an iteration; element by element it does not.  TL_SOLVER_AUTO takes a single
+  // body whose longest chain is over HUB_SLOTS element by element.  A step of 2,730 nodes, FP64: widest row 27 0.79 ms
+  // for 0.95, 57 (a chain of 57) 1.59 for 1.07; of 1,000 nodes, 99 (25) 0.85 for 1.07, 153 (39) 1.23 for 1.22; of 8,000
+  // in kPcgSell 27 1.32 for 1.33, 57 2.33 for 1.40; of a 12,153-node fan around one node 497 for 16.
+  static constexpr uint32_t HUB_SLOTS = 32;
+  bool sellHub = false;
+  bool hubForm() const { return sellHub && solverForm == TL_SOLVER_AUTO; }
   // The body's rows over the blocks of one cluster (kPcgCluster).
   struct ClusterPlan {
     const void* kernel = nullptr;  // null: none
@@ -1081,7 +1090,8 @@ struct System final : SystemBase {
   }
   // Whether this system's solves run in a cluster.
   bool clusterForm() const {
-    return sellReady && cluster.kernel && (solverForm == TL_SOLVER_AUTO || solverForm == TL_SOLVER_ASSEMBLED);
+    return sellReady && cluster.kernel && !hubForm() &&
+           (solverForm == TL_SOLVER_AUTO || solverForm == TL_SOLVER_ASSEMBLED);
   }
   // Shared memory of kPcgSell: its first columns and the blocks of its first slots.
   uint32_t sellKept = 0;
@@ -1124,7 +1134,7 @@ struct System final : SystemBase {
   // Whether this system's PCG may run on the assembled matrix, which TL_SOLVER_AUTO chooses wherever kPcgCluster or
   // kPcgSell takes the bodies: with one block per SM kPcgSell overtakes the element-by-element kernel for every body past a cluster's (5,202 nodes, a frame: 1.19
   // against 1.38 ms in FP32-mixed, 1.40 against 1.59 in FP64, the assembly included).
-  bool assembledForm() const { return sellReady && solverForm != TL_SOLVER_ELEMENTWISE; }
+  bool assembledForm() const { return sellReady && solverForm != TL_SOLVER_ELEMENTWISE && !hubForm(); }
   // Whether a solve that kPcgSell does not take runs in one of the lockstep orders.  A single body of more rows than the
   // resident grid has threads keeps the element-by-element route in TL_SOLVER_AUTO.  ASSEMBLED asks for the lockstep one
   // (two steps at the default settings, 91,908 nodes: FP64 17.4 ms element by element, 16.1 assembled, FP32-mixed 9.5
