@@ -1030,7 +1030,12 @@ struct System final : SystemBase {
   // One body whose rows fit the blocks of a cluster of 16: up to 10 slices a block, 5,120 rows.  At 4,624 rows an
   // iteration takes 7.0 us where the whole-GPU kernels take 7.7 (FP32-mixed) and 9.0 us (FP64), at 3,840 4.9
   // against 7.7 and 8.9, at 1,331 2.3 against 7.5 and 8.4.  More rows find no worker for every slice and fewer of
-  // their blocks on the SM.  16 blocks beat 8 and 4 from 250 rows up and equal them below.
+  // their blocks on the SM.  16 blocks beat 8 and 4 from 250 rows up and equal them below.  A foreign entry costs a block
+  // 2.9 ns an iteration, so nodes in no order of place (a lattice of 5,120 nodes has 640 foreign entries in a block, in
+  // random order 2,714) go to kPcgSell above CLUSTER_FOREIGN: a step
+  // of 4,352 such nodes 1.37 ms here and 0.98 there (FP32-mixed 1.32 and 0.86), of 2,730 (1,531 entries) 0.86 and 0.92
+  // (0.85 and 0.83).
+  static constexpr uint32_t CLUSTER_FOREIGN = 1536;
   void buildCluster(const SellHost& h) {
     cluster = ClusterPlan{};
     if (B != 1) return;
@@ -1040,6 +1045,7 @@ struct System final : SystemBase {
     if (owners > CLUSTER_OWNERS || perBlock > CLUSTER_W - owners) return;  // a worker for every slice
     ClusterHost c;
     if (!buildClusterHost(h, CLUSTER_MAX, c)) return;
+    if (*std::max_element(c.foreign.begin(), c.foreign.end()) > CLUSTER_FOREIGN) return;
     ClusterDev& d = cluster.dev;
     d.slices = perBlock;
     d.owners = owners;

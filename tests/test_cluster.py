@@ -169,3 +169,35 @@ def test_operator_applications_are_those_of_the_elementwise_form(cells):
         out[form] = [(r.cg_iterations, r.operator_applications) for r in reports]
         s.close()
     assert out["auto"] == out["elementwise"]
+
+
+def scattered(mesh, share, seed):
+    """The mesh with a share of its nodes renumbered among themselves."""
+    order = np.arange(mesh.nodes)
+    some = np.random.default_rng(seed).permutation(mesh.nodes)[:int(share * mesh.nodes)]
+    order[np.sort(some)] = some
+    rank = np.argsort(order)
+    return tb.PreparedMesh(mesh.rest_positions[order], mesh.node_mass[order], mesh.anchored[order],
+                           rank[mesh.tet_nodes].astype(np.uint32), mesh.rest_inverse, mesh.volume, mesh.material)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells,share,cluster", [((15, 16, 15), 0.0, True), ((15, 16, 15), 0.1, True),
+                                                 ((15, 16, 15), 1.0, False), ((9, 9, 9), 1.0, True)])
+@pytest.mark.parametrize("precision,tol", [(tb.FP64, 1e-10), (tb.FP32_MIXED, 1e-5)])
+def test_nodes_in_no_order_of_place(cells, share, cluster, precision, tol):
+    """A body whose blocks read too many foreign rows solves over the whole grid, which takes one more launch a solve;
+    one with a tenth of its nodes scattered (rows that more than four blocks read) stays in the cluster."""
+    mesh = scattered(tb.box_mesh(cells, voxel=0.1, jitter=0.01, seed=3), share, 2)
+    mat = tb.PhysicalMaterial(density=1000.0, youngs_modulus=1e6, poissons_ratio=0.3)
+    out = {}
+    for form in ("auto", "assembled-two-phase", "elementwise"):
+        s = tb.System(mesh, [mat], precision)
+        s.set_solver(form)
+        s.set_state(tb.rest_state(mesh))
+        reports = [s.step(tb.Settings(), GRAVITY, DT)[0] for _ in range(2)]
+        out[form] = s.get_state().position, reports[-1]
+        s.close()
+    launches = {f: r.kernel_launches for f, (_, r) in out.items()}
+    assert (launches["auto"] < launches["assembled-two-phase"]) == cluster
+    assert relative_error(out["auto"][0], out["elementwise"][0], mesh.rest_positions) <= tol
