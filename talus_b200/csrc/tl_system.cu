@@ -983,7 +983,7 @@ struct System final : SystemBase {
       }
     }
     tuneRowGroup = held;
-    sellPerSm = sellPerSmOf[sellU() == 4u ? 1 : 0];
+    sellPerSm = std::min(sellPerSmOf[0], sellPerSmOf[1]);  // the same parts, and so the same sums, for both row groups
     buildGang();
     // kPcgBatchSell: every batch, and single bodies whose rows exceed one per thread of kPcgSell's grid
     sellP2.alloc(Vp);
@@ -2591,7 +2591,6 @@ struct System final : SystemBase {
       throw StatusError{TL_ERR_ARG, "no such launch-shape knob"};
     }
     if (sellReady) {
-      sellPerSm = sellPerSmOf[sellU() == 4u ? 1 : 0];
       batchSellPerSm = occupancyOf(batchKernel(true), 0);
       batchPipePerSm = occupancyOf(batchKernel(false), 0);
       if (batchSellPerSm < 1 || batchPipePerSm < 1) throw StatusError{TL_ERR_CUDA, "shape cannot be resident"};

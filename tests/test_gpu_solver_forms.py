@@ -220,3 +220,24 @@ def test_assembled_forms_of_a_body_too_large_for_one_row_per_thread(form, precis
     assert [r["kernel_launches"] - r["cg_solves"] for r in ra] == [r["kernel_launches"] for r in re]
     if precision == tb.FP64:
         assert [r["cg_iterations"] for r in ra] == [r["cg_iterations"] for r in re]
+
+
+# bodies past a cluster's size: over less than the grid, with a block per SM, with two; a batch in one queue
+@pytest.mark.parametrize("cells", [[(16, 16, 17)], [(34, 31, 30)], [(48, 28, 29)], [(9, 7, 8), (3, 3, 3), (12, 11, 10)]])
+@pytest.mark.parametrize("precision", [tb.FP64, tb.FP32_MIXED])
+def test_row_groups_give_bitwise_the_same_step_over_the_grid(cells, precision):
+    """kPcgSell adds a row's slots in order and a body's partials by its parts, whatever the row group."""
+    meshes = [tb.box_mesh(c, voxel=0.1, jitter=0.01, seed=4) for c in cells]
+    mats = [[tb.PhysicalMaterial(density=1000.0, youngs_modulus=1e6, poissons_ratio=0.3)] for _ in meshes]
+    results = []
+    for row_group in (0, 2, 4):
+        s = tb.System(meshes, mats, precision)
+        s.tune_shape(row_group)
+        for i, m in enumerate(meshes):
+            s.set_state(tb.rest_state(m), i)
+        for _ in range(2):
+            s.step(tb.Settings(), GRAVITY, DT)
+        results.append(np.concatenate([s.get_state(i).position.ravel() for i in range(len(meshes))]))
+        s.close()
+    for r in results[1:]:
+        assert np.array_equal(r, results[0])
