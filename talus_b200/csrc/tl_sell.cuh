@@ -428,10 +428,11 @@ template <class S> __device__ __forceinline__ V3<double> roundTo(V3<double> v) {
 // above 1e-6 in FP32-mixed on the breakdown test, the worst at 1e-3, and a
 // layered body (stiffnesses 1e4 apart) at 0.3; with it none does, and they take
 // as many iterations as the textbook order (34,989 for 35,684 before in a frame
-// of those bodies: 32.0 ms for 32.2; FP64 steps of 166,050 tets take 8.07
-// ms for 7.89, FP32-mixed ones of 393,216 tets 9.5 for 9.8, as unpacking is
-// cheaper than converting).
-// The steps are written out in FP64 and a loop in FP32-mixed, as each spills least.
+// of those bodies: 32.2 ms as before).  It costs no time where it does not
+// fire: two FP64 frames of 166,050 tets 7.8 ms for 7.9, of 48,000 5.7 for 6.0,
+// two FP32-mixed ones of 393,216 tets 9.5 for 9.7, as unpacking is cheaper than
+// converting.  The steps are written out in an FP64 batch and a loop elsewhere,
+// as each spills least.
 constexpr int SELL_FALL = 23 << 20;  // a factor of 2^-23, in the upper word of a double
 template <class S, bool GANG, uint32_t U>
 __global__ void __launch_bounds__(TILE, 2)
@@ -539,26 +540,53 @@ __global__ void __launch_bounds__(TILE, 2)
     double sums[4];
     sumBlocksAll<4>(part4, sums, G);
     double gammaNext = sums[0], delta = sums[1], length = sums[2];
-    double target = 0.0;
-    {
-      const double floor = fmax(sqrt(sums[3]), 1.1754943508222875e-38);  // std::numeric_limits<float>::min()
-      target = st.tolerance * floor;
-      if (part == 0 && threadIdx.x == 0) {
-        s.cg[b].floor = floor;
-        s.cg[b].start_res = sqrt(length) / floor;
-      }
+    const double floor = fmax(sqrt(sums[3]), 1.1754943508222875e-38);  // std::numeric_limits<float>::min()
+    const double target = st.tolerance * floor;
+    const double startRes = sqrt(length) / floor;
+    if (GANG && part == 0 && threadIdx.x == 0) {  // where the queue's variables leave no registers for them
+      s.cg[b].floor = floor;
+      s.cg[b].start_res = startRes;
     }
     double gamma = 0.0, alpha = 0.0, beta = 0.0;
     uint32_t taken = 0;
     V3<double> zv = {0, 0, 0}, qv = {0, 0, 0}, sv = {0, 0, 0}, pv = {0, 0, 0};
     int mostLength = 0, mostGamma = 0;  // upper words of the largest since the last replacement
     bool fresh = true;                  // no update since then
+    // m = P w published, the sums, n = A m; false when a wait ran out
+    const auto advance = [&]() {
+      m = precondition(w);
+      if (mine) vec()[row] = publishedOf<S>(m);
+      double* const mine_part = partials();
+      {
+        double v[3] = {dot(r, u), dot(w, u), dot(r, r)};
+        blockSum<3>(v);
+        if (threadIdx.x == 0)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) mine_part[k * G + part] = v[k];
+      }
+      if (!gangBarrier(arrive, G, s.sync, bar)) return false;
+      // n = A m for the next iteration, with the block partials requested first so that both round trips overlap
+      if (stagedSums) requestBlockPartials(mine_part, partStage, 3u, G);
+      n = product();
+      double d[3];
+      if (stagedSums) {
+        cpAsyncWaitAll();
+        __syncthreads();
+        sumStagedBlocks<3>(partStage, d, G);
+      } else {
+        sumBlocksAll<3>(mine_part, d, G);
+      }
+      gammaNext = d[0];
+      delta = d[1];
+      length = d[2];
+      return true;
+    };
     for (;;) {
       if (taken >= st.limit || sqrt(length) <= target) break;  // the reference's loop-top test
       mostLength = max(fresh ? 0 : mostLength, __double2hiint(length));
       mostGamma = max(fresh ? 0 : mostGamma, __double2hiint(gammaNext));
       if (!fresh && (__double2hiint(length) < mostLength - SELL_FALL || __double2hiint(gammaNext) < mostGamma - SELL_FALL)) {
-        constexpr int copies = sizeof(S) == 8 ? 4 : 1;
+        constexpr int copies = sizeof(S) == 8 && GANG ? 4 : 1;
         // x (FP64), p, P r and P s published in turn: r = right - A x, s = A p, w = A u, z = A q
 #pragma unroll copies
         for (uint32_t k = sizeof(S) == 8 ? 0u : 1u; k < 4u; ++k) {
@@ -581,6 +609,10 @@ __global__ void __launch_bounds__(TILE, 2)
         }
         if (threadIdx.x == 0) extra += sizeof(S) == 8 ? 4u : 3u;
         fresh = true;
+        if constexpr (!GANG) {  // apart from the update's, which so stays a straight line (FP64, 9,261 nodes: 4% of a step)
+          if (!advance()) return;
+          continue;
+        }
       } else {
         const double bl = taken ? gammaNext / gamma : 0.0;
         const double curvature = taken ? delta - bl * gammaNext / alpha : delta;  // p.A p
@@ -617,36 +649,14 @@ __global__ void __launch_bounds__(TILE, 2)
         ++taken;
         fresh = false;
       }
-      m = precondition(w);
-      if (mine) vec()[row] = publishedOf<S>(m);
-      double* const mine_part = partials();
-      {
-        double v[3] = {dot(r, u), dot(w, u), dot(r, r)};
-        blockSum<3>(v);
-        if (threadIdx.x == 0)
-#pragma unroll
-          for (int k = 0; k < 3; ++k) mine_part[k * G + part] = v[k];
-      }
-      if (!gangBarrier(arrive, G, s.sync, bar)) return;
-      // n = A m for the next iteration, with the block partials requested first so that both round trips overlap
-      if (stagedSums) requestBlockPartials(mine_part, partStage, 3u, G);
-      n = product();
-      double d[3];
-      if (stagedSums) {
-        cpAsyncWaitAll();
-        __syncthreads();
-        sumStagedBlocks<3>(partStage, d, G);
-      } else {
-        sumBlocksAll<3>(mine_part, d, G);
-      }
-      gammaNext = d[0];
-      delta = d[1];
-      length = d[2];
+      if (!advance()) return;
     }
     if (live) X[row] = pack(cvt<S>(x));
     if (part == 0 && threadIdx.x == 0) {
       const double residual = sqrt(length);
-      CgBodyDev c = s.cg[b];  // floor and start_res as written at the start
+      CgBodyDev c;
+      c.floor = GANG ? s.cg[b].floor : floor;
+      c.start_res = GANG ? s.cg[b].start_res : startRes;
       c.squared = gamma;
       c.target = target;
       c.length = length;
