@@ -165,8 +165,6 @@ def pcg_bytes_per_iteration(T, V, slots, s_bytes, tangent):
     return a + b + c
 
 
-
-
 def operator_blocks(mesh):
     """Nonzero 3x3 blocks of the assembled single-body operator: the ordered
     node pairs that share an element (the diagonal included)."""
@@ -175,23 +173,52 @@ def operator_blocks(mesh):
     return int(np.unique(pairs).size)
 
 
-def sell_bytes_per_iteration(blocks, V, s_bytes):
-    """Unique bytes of one tl::kPcgSell iteration (talus_b200/csrc/tl_sell.cuh):
-    every block of the matrix (9 S entries and its column index) and the
-    published matvec input read once, the next input written once.  The
-    iteration vectors stay in registers."""
+def assembled_bytes_per_iteration(kernel, blocks, V, s_bytes):
+    """Unique bytes of one body's iteration on the assembled matrix, by the
+    kernel that ran: every block (9 S entries and its column index) once, and
+    per node
+      kPcgSell           the published matvec input read and the next one
+                         written; the vectors stay in registers;
+      kPcgBatchSell      the previous direction and z gathered, the new
+                         direction and A p written (phase AB), then direction,
+                         x, A p, r and the preconditioner (2 records) read and
+                         x, r, z written (phase C);
+      kPcgBatchSellPipe  the input read and written, the eight FP64 planes read
+                         and written, the preconditioner read, and X written
+                         in FP32-mixed.
+    kPcgCluster keeps matrix and vectors on the chip: no bytes but those of the
+    solve's start, which are the matrix once."""
     v4 = 4 * s_bytes
-    return blocks * (9 * s_bytes + 4) + 2 * V * v4
+    matrix = blocks * (9 * s_bytes + 4)
+    if kernel == "kPcgCluster":
+        return 0
+    if kernel == "kPcgSell":
+        return matrix + V * 2 * v4
+    if kernel == "kPcgBatchSell":
+        return matrix + V * 13 * v4
+    return matrix + V * (4 * v4 + 16 * 32 + (v4 if s_bytes == 4 else 0))
 
 
-def sell_batch_bytes_per_iteration(blocks, V, s_bytes):
-    """Unique bytes of one body's iteration in tl::kPcgBatchSell: the body's
-    matrix blocks (9 S entries and a column index) once; per node, the
-    previous direction and z gathered, the new direction and A p written
-    (phase AB), then direction, x, A p, r, the preconditioner (2 records)
-    read and x, r, z written (phase C)."""
-    v4 = 4 * s_bytes
-    return blocks * (9 * s_bytes + 4) + V * 13 * v4
+# where the bytes of an iteration come from: a matrix that a solve holds on the
+# chip (registers, shared memory, the 126 MB L2) has no HBM bound per iteration
+PCG_KERNELS = {
+    "kPcgCluster": "persistent block-Jacobi PCG of one body inside one thread-block cluster, matrix on the chip",
+    "kPcgSell": "persistent pipelined block-Jacobi PCG on the assembled sliced-ELL block matrix, "
+                "each body iterated by its own blocks",
+    "kPcgBatchSell": "persistent block-Jacobi PCG in lockstep on the assembled block matrix, two-phase order",
+    "kPcgBatchSellPipe": "persistent block-Jacobi PCG in lockstep on the assembled block matrix, pipelined order",
+    "kPcg1": "persistent block-Jacobi PCG, element by element, two-level assembly",
+    "kPcgBatch": "persistent block-Jacobi PCG over all bodies, element by element",
+}
+
+
+def pcg_bound(kernel, matrix_bytes):
+    """What limits an iteration: kPcgCluster's exchanges; for kPcgSell, whose
+    bodies in work hold at most 75,776 rows, and for a lockstep matrix that
+    fits it, the L2; otherwise HBM."""
+    if kernel == "kPcgCluster":
+        return "latency"
+    return "l2" if kernel == "kPcgSell" or matrix_bytes < 126e6 else "hbm"
 
 
 def sell_assembly_bytes(T, blocks, s_bytes, tangent):
@@ -538,15 +565,17 @@ def run_ours(args, spec, rank, world, dist):
     s_bytes = 4 if precision == tb.FP32_MIXED else 8
     pcg_bytes = 0.0
     assembly = None
-    # the form the system took (TL_SOLVER_AUTO: assembled)
-    form = tune.get("solver", "auto") if tune else "auto"
-    assembled = form != "elementwise"
+    kernel = system.pcg_kernel()  # the one the steps ran
+    assembled = kernel not in ("kPcg1", "kPcgBatch")
+    matrix_bytes = 0.0
     for b, m in enumerate(meshes):
         it, tan = per_body[b, 0], per_body[b, 1]
         if assembled:  # assembled operator (tl_sell.cuh)
             blocks = operator_blocks(m)
-            per_it = (sell_bytes_per_iteration if B == 1 else sell_batch_bytes_per_iteration)(blocks, m.nodes, s_bytes)
-            pcg_bytes += per_it * it
+            matrix_bytes += blocks * (9 * s_bytes + 4)
+            pcg_bytes += assembled_bytes_per_iteration(kernel, blocks, m.nodes, s_bytes) * it
+            if kernel == "kPcgCluster":
+                pcg_bytes += blocks * (9 * s_bytes + 4) * per_body[b, 2]
             if assembly is None:
                 assembly = {"kernel": "tl::kSellAssemble (block matrix, once per solve)", "blocks": 0,
                             "algorithmic_bytes_per_launch": 0}
@@ -565,17 +594,10 @@ def run_ours(args, spec, rank, world, dist):
     if os.path.exists(tpath):
         with open(tpath) as f:
             tr = json.load(f)
-        prefix = ("tl::kPcgSell" if B == 1 else "tl::kPcgBatchSell") if assembled else (
-            "tl::kPcg1" if B == 1 else "tl::kPcgBatch<")
-        same_kernel = tr.get("kernel", "").startswith(prefix)
+        same_kernel = tr.get("kernel", "").startswith(f"tl::{kernel}<")
         if tr.get("workload") == args.workload and tr.get("precision") == args.precision and same_kernel and launches_pcg:
             traffic = tr["dram_bytes_per_iteration"] * per_body[:, 0].sum() / launches_pcg
 
-    if B == 1:
-        kernel = ("tl::kPcgSell (persistent pipelined block-Jacobi PCG on the assembled sliced-ELL block matrix)"
-                  if assembled else "tl::kPcg1 (persistent block-Jacobi PCG, element by element, two-level assembly)")
-    else:
-        kernel = "tl::kPcgBatchSell (persistent block-Jacobi PCG over all bodies on the assembled block matrix)"
     config = {"workload": args.workload, "bodies": B, "tets": T, "nodes": V, "law": spec["law"],
               "precision": args.precision, "dt": 1.0 / 60.0,
               "parallelism": "single-gpu" if world == 1 else (f"shards{world}" if spec.get("batch") else f"replicas{world}"),
@@ -599,7 +621,8 @@ def run_ours(args, spec, rank, world, dist):
                 "steps": e2e_steps,
                 "api": ("tl_step_host" if B == 1 else "tl_state_set + tl_step + tl_state_get") + " (state in host memory, f32, buffers page-locked once by tl_host_register)"},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": kernel, "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"bound": pcg_bound(kernel, matrix_bytes) if assembled else "hbm",
+                     "kernel": f"tl::{kernel} ({PCG_KERNELS[kernel]})", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": traffic, "launches": launches_pcg,
                      "iterations": int(per_body[:, 0].max()),
                      "algorithmic_bytes_per_launch": pcg_bytes / max(1, launches_pcg),
@@ -852,6 +875,7 @@ def batch_form(context, flush, warmup=2, steps=5, tolerance=1e-6, cap=4000):
             system.step(settings)
         seconds, iters, launches, capped = 0.0, [], 0, 0
         body_iters = np.zeros(len(meshes))
+        residual = 0.0
         for _ in range(steps):
             flush.zero_()
             torch.cuda.synchronize()
@@ -861,25 +885,27 @@ def batch_form(context, flush, warmup=2, steps=5, tolerance=1e-6, cap=4000):
             iters.append(max(r.cg_iterations for r in reps))
             body_iters += [r.cg_iterations for r in reps]
             capped += sum(r.cg_capped_solves for r in reps)
+            residual = max(residual, *(r.cg_worst_relative_residual for r in reps))
         finals[name] = [system.get_state(i).position for i in range(len(meshes))]
-        # one more step with per-class device times: the batched PCG against its algorithmic bytes
-        # (per body-iteration: blocks (9s + 4) for the matrix and its columns, plus the node vectors
-        # each order moves: 13 (two-phase) or 19 (pipelined) four-wide vectors of s bytes)
+        # one more step with per-class device times: the bytes that the PCG's iterations use, by the kernel that ran
         flush.zero_()
         torch.cuda.synchronize()
         preps = system.step(tb.Settings(cg_iterations=cap, tolerance=tolerance, profile=True))
         s_bytes = 4 if precision == tb.FP32_MIXED else 8
-        form = (tune or {}).get("solver", "auto")
-        piped = form == "assembled-pipelined" or (form in ("auto", "assembled") and precision == tb.FP64)
-        vectors = 19 if piped else 13
-        pcg_bytes = float(sum(r.cg_iterations * (blocks[i] * (9 * s_bytes + 4) + m.nodes * vectors * 4 * s_bytes)
-                              for i, (r, m) in enumerate(zip(preps, meshes))))
+        kernel = system.pcg_kernel()
+        if kernel == "kPcgBatch":  # element by element
+            pcg_bytes = float(sum(r.cg_iterations * pcg_bytes_per_iteration(m.tets, m.nodes, tile_slots(m), s_bytes, False)
+                                  for r, m in zip(preps, meshes)))
+        else:
+            pcg_bytes = float(sum(r.cg_iterations * assembled_bytes_per_iteration(kernel, k, m.nodes, s_bytes)
+                                  for r, k, m in zip(preps, blocks, meshes)))
         pcg_s = preps[0].pcg_seconds
         peak, peak_kind = peaks()
-        pcg_roof = {"kernel": "tl::kPcgBatchSellPipe" if piped else "tl::kPcgBatchSell",
+        pcg_roof = {"kernel": f"tl::{kernel}", "bound": pcg_bound(kernel, sum(blocks) * (9 * s_bytes + 4)),
                     "algorithmic_bytes_per_step": pcg_bytes, "pcg_ms_per_step": pcg_s * 1e3,
                     "achieved": pcg_bytes / pcg_s / 1e9 if pcg_s > 0 else None, "peak": peak, "unit": "GB/s",
                     "frac": pcg_bytes / pcg_s / 1e9 / peak if pcg_s > 0 else None, "peak_kind": peak_kind,
+                    "note": "peak is HBM's; bytes that an iteration finds in L2 or shared memory are not bound by it",
                     "step_ms_with_events": preps[0].device_seconds * 1e3}
         system.close()
         tets = sum(m.tets for m in meshes)
@@ -888,7 +914,8 @@ def batch_form(context, flush, warmup=2, steps=5, tolerance=1e-6, cap=4000):
                      "body_cg_iterations_per_step": {
                          q: float(np.percentile(body_iters / steps, p)) for q, p in
                          (("min", 0), ("median", 50), ("p90", 90), ("max", 100))},
-                     "capped_solves": capped, "tuning": tune, "pcg_roofline": pcg_roof}
+                     "capped_solves": capped, "worst_relative_residual": residual, "tuning": tune,
+                     "pcg_roofline": pcg_roof}
     worst = max(float(np.linalg.norm(a - b, axis=1).max() / np.linalg.norm(b - m.rest_positions, axis=1).max())
                 for a, b, m in zip(finals["mixed"], finals["fp64"], meshes))
     return {"workload": f"batch, {len(meshes)} bodies, {sum(m.tets for m in meshes)} tets", "unit": UNIT,

@@ -227,6 +227,13 @@ int32_t tl_system_tune_shape(tl_system* system, uint32_t knob, uint32_t value);
 #define TL_SOLVER_ASSEMBLED_PIPELINED 4u
 int32_t tl_system_set_solver(tl_system* system, uint32_t form);
 
+/* Diagnostics, no reference counterpart: the kernel that the system's next
+ * PCG solves run in with its present form ("kPcgCluster", "kPcgSell",
+ * "kPcgBatchSell", "kPcgBatchSellPipe", "kPcg1", "kPcgBatch"; with a solver
+ * state's factor on the device "kPcgInverse" or "kPcgFactor").  *name is a
+ * constant of the library. */
+int32_t tl_system_pcg_kernel(const tl_system* system, const char** name);
+
 /* The caller-held solver state of deformable::step (DeformableSolverState*,
  * factor.h:205-210; solver.cc:3606-3655, 3808-3910, 4258-4263), held by the
  * library for a one-body system.  While it is on, every step preconditions

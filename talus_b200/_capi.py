@@ -172,6 +172,7 @@ SIGNATURES = {
     "tl_host_register": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_size_t]),
     "tl_host_unregister": (C.c_int32, [C.c_void_p, C.c_void_p]),
     "tl_system_set_solver": (C.c_int32, [C.c_void_p, C.c_uint32]),
+    "tl_system_pcg_kernel": (C.c_int32, [C.c_void_p, C.POINTER(C.c_char_p)]),
     "tl_system_use_factor": (C.c_int32, [C.c_void_p, C.c_uint32, C.c_uint32]),
     "tl_system_factor_stats": (C.c_int32, [C.c_void_p, C.POINTER(tl_factor_stats)]),
     "tl_system_set_plasticity": (C.c_int32, [C.c_void_p, C.c_uint32]),

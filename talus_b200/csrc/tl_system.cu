@@ -261,6 +261,7 @@ struct SystemBase {
   virtual void tune(uint32_t blocksPerSm, uint32_t graph) = 0;
   virtual void tuneShape(uint32_t knob, uint32_t value) = 0;
   virtual void setSolver(uint32_t form) = 0;
+  virtual const char* pcgKernel() const = 0;
   virtual void useFactor(uint32_t enable, uint32_t budget) = 0;
   virtual void factorStats(tl_factor_stats* out) = 0;
   virtual void setPlasticity(uint32_t mode) = 0;
@@ -1148,6 +1149,20 @@ struct System final : SystemBase {
   bool lockstepForm() const {
     return assembledForm() && batchSellPerSm > 0 && (B > 1 || solverForm != TL_SOLVER_AUTO);
   }
+  // The lockstep order that is taken where none is asked for.  FP32-mixed: the faster one (two steps of a 91,908-node
+  // body and 20 of 1,000 nodes, two-phase against pipelined: 10.6 and 13.2 ms at the default settings, 26.5 and 32.5 to
+  // 1e-6).  FP64: the two are within 2% there (19.4 and 19.6, 49.5 and 50.5), and the pipelined order is 8% faster for
+  // such a body alone (17.5 and 16.1).
+  bool twoPhaseForm() const {
+    return solverForm == TL_SOLVER_ASSEMBLED_TWO_PHASE || (solverForm != TL_SOLVER_ASSEMBLED_PIPELINED && sizeof(S) == 4);
+  }
+  const char* pcgKernel() const override {
+    if (factorOn && dfReady) return fInverse ? "kPcgInverse" : "kPcgFactor";
+    if (clusterForm()) return "kPcgCluster";
+    if (sellGrid() > 0) return "kPcgSell";
+    if (lockstepForm()) return twoPhaseForm() ? "kPcgBatchSell" : "kPcgBatchSellPipe";
+    return B == 1 ? "kPcg1" : "kPcgBatch";
+  }
   // Grid of kPcgSell, or 0 where it does not run: a body with more rows than the grid has threads, or a batch in one
   // of the lockstep orders.
   int sellGrid() const {
@@ -1675,11 +1690,7 @@ struct System final : SystemBase {
         mark(2, true);
       }
       Vec4<S>* p2 = sellP2.ptr;
-      // FP32-mixed: the faster order (two steps of a 91,908-node body and 20 of 1,000 nodes, two-phase against pipelined:
-      // 10.6 and 13.2 ms at the default settings, 26.5 and 32.5 to 1e-6).  FP64: the two are within 2% there (19.4 and
-      // 19.6, 49.5 and 50.5), and the pipelined order is 8% faster for such a body alone (17.5 and 16.1)
-      const bool twoPhase = solverForm == TL_SOLVER_ASSEMBLED_TWO_PHASE ||
-                            (solverForm != TL_SOLVER_ASSEMBLED_PIPELINED && sizeof(S) == 4);
+      const bool twoPhase = twoPhaseForm();
       int perSm = twoPhase ? batchSellPerSm : batchPipePerSm;
       int grid = std::max(1, std::min(perSm * ctx->sms, int(nodeTiles)));
       // the block's slot table: body and row count of each of its tiles
@@ -3546,6 +3557,12 @@ int32_t tl_system_set_solver(tl_system* system, uint32_t form) {
     system->impl->setSolver(form);
     return TL_OK;
   });
+}
+
+int32_t tl_system_pcg_kernel(const tl_system* system, const char** name) {
+  if (!system || !name) return TL_ERR_ARG;
+  *name = system->impl->pcgKernel();
+  return TL_OK;
 }
 
 int32_t tl_system_use_factor(tl_system* system, uint32_t enable, uint32_t factor_budget) {

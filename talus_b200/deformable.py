@@ -292,6 +292,12 @@ class System:
         check(capi.lib().tl_system_factor_stats(self.handle, C.byref(out)), self.context.handle)
         return out.as_dict()
 
+    def pcg_kernel(self) -> str:
+        """The kernel the next PCG solves run in (tl_system_pcg_kernel)."""
+        name = C.c_char_p()
+        check(capi.lib().tl_system_pcg_kernel(self.handle, C.byref(name)), self.context.handle)
+        return name.value.decode()
+
     def factor_form(self):
         """How the solver state's factor is applied (tl_factor_stats::form):
         "inverse", "lean", or None before one is made."""

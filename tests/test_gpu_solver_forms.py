@@ -241,3 +241,28 @@ def test_row_groups_give_bitwise_the_same_step_over_the_grid(cells, precision):
         s.close()
     for r in results[1:]:
         assert np.array_equal(r, results[0])
+
+
+def test_the_kernel_that_runs_is_reported():
+    small, mat = elastic_block((4, 4, 4))
+    mid, big = tb.box_mesh((16, 16, 17), voxel=0.1), tb.box_mesh((68, 36, 35), voxel=0.1)
+    forms = ("auto", "assembled", "assembled-two-phase", "assembled-pipelined", "elementwise")
+    expected = {
+        "small": ("kPcgCluster", "kPcgCluster", "kPcgSell", "kPcgSell", "kPcg1"),
+        "mid": ("kPcgSell", "kPcgSell", "kPcgSell", "kPcgSell", "kPcg1"),
+        "big": ("kPcg1", "kPcgBatchSellPipe", "kPcgBatchSell", "kPcgBatchSellPipe", "kPcg1"),
+        "batch": ("kPcgSell", "kPcgSell", "kPcgBatchSell", "kPcgBatchSellPipe", "kPcgBatch"),
+        "batch with big": ("kPcgBatchSellPipe", "kPcgBatchSellPipe", "kPcgBatchSell", "kPcgBatchSellPipe", "kPcgBatch"),
+    }
+    for name, meshes in (("small", [small]), ("mid", [mid]), ("big", [big]), ("batch", [small, mid]),
+                         ("batch with big", [small, big])):
+        s = tb.System(meshes, [[mat] for _ in meshes], tb.FP64)
+        got = []
+        for form in forms:
+            s.set_solver(form)
+            got.append(s.pcg_kernel())
+        assert tuple(got) == expected[name], name
+        s.close()
+    s = tb.System([small, big], [[mat], [mat]], tb.FP32_MIXED)
+    assert s.pcg_kernel() == "kPcgBatchSell"
+    s.close()
