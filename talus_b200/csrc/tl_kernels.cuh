@@ -143,7 +143,7 @@ struct GridSyncDev {
   int error;
   int active;      // bodies still iterating in the current PCG solve
   int active_odd;  // its copy for odd phases of the one-barrier batched PCG (kPcgBatchSellPipe)
-  unsigned int ticket;  // bodies handed out to the clusters of kPcgCluster beyond their first
+  unsigned int ticket;  // items of kPcgSell's queue handed out beyond each block's first
 };
 
 // Per-element matvec operator, one record per element: the gradients
