@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import talus_b200 as tb
-from tests.helpers import DT, GRAVITY
+from tests.helpers import DT, GRAVITY, plastic_block
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +80,21 @@ def test_lockstep_pipelined_batch(precision, tolerance):
     meshes = [tb.box_mesh(c, voxel=0.1) for c in ((12, 11, 10), (3, 30, 4), (2, 2, 2), (9, 20, 9), (7, 7, 3))]
     mats = [[material(e, 0.35)] for e in (1e8, 3e7, 1e5, 1e8, 1e6)]
     check(stepped(meshes, mats, precision, tolerance, "assembled-pipelined"), tolerance)
+
+
+def test_floating_body_at_the_default_settings():
+    """A floating body solves to 1e-5 whatever the settings ask, in FP32-mixed too."""
+    mesh = tb.box_mesh((17, 17, 17), voxel=0.1, jitter=0.01, seed=4, anchor_axis=3)
+    check(stepped(mesh, [material(1e8)], tb.FP32_MIXED, 1e-3, "auto"), 1e-5)
+
+
+@pytest.mark.parametrize("precision,tolerance", [(tb.FP32_MIXED, 1e-6), (tb.FP64, 1e-11)])
+def test_yielding_body(precision, tolerance):
+    """The plastic Newton loop's solves, with the consistent operator among them."""
+    mesh, mat = plastic_block((18, 17, 17), speed=4.0)
+    s = tb.System(mesh, [mat], precision)
+    s.set_state(tb.rest_state(mesh))
+    reports = [s.step(tb.Settings(tolerance=tolerance, cg_iterations=4000), GRAVITY, DT) for _ in range(3)]
+    s.close()
+    assert any(r[0].cg_tangent_iterations > 0 for r in reports)
+    check(reports, tolerance)
