@@ -300,7 +300,8 @@ __device__ __forceinline__ void sellNear(const S* v, V xin, V3<double>& acc) {
 // per round trip, the blocks of its first `kept` slots (a multiple of U) from
 // shared memory.
 template <class S, uint32_t U, class V>
-__device__ __forceinline__ V3<double> sellRow(const SellDev<S>& g, uint32_t slice, uint32_t lane, const V* in, const uint32_t* cols, const S* near, uint32_t kept) {
+__device__ __forceinline__ V3<double> sellRow(const SellDev<S>& g, uint32_t slice, uint32_t lane, const V* in,
+                                              const uint32_t* cols, const S* near, uint32_t kept) {
   V3<double> acc = {0, 0, 0};
   const uint32_t p1 = __ldg(&g.slice_start[slice + 1]);
   uint32_t p = __ldg(&g.slice_start[slice]) + lane, k = 0;
@@ -585,7 +586,8 @@ __global__ void __launch_bounds__(TILE, 2)
       if (taken >= st.limit || sqrt(length) <= target) break;  // the reference's loop-top test
       mostLength = max(fresh ? 0 : mostLength, __double2hiint(length));
       mostGamma = max(fresh ? 0 : mostGamma, __double2hiint(gammaNext));
-      if (!fresh && (__double2hiint(length) < mostLength - SELL_FALL || __double2hiint(gammaNext) < mostGamma - SELL_FALL)) {
+      if (!fresh && (__double2hiint(length) < mostLength - SELL_FALL ||
+                     __double2hiint(gammaNext) < mostGamma - SELL_FALL)) {
         constexpr int copies = sizeof(S) == 8 && GANG ? 4 : 1;
         // x (FP64), p, P r and P s published in turn: r = right - A x, s = A p, w = A u, z = A q
 #pragma unroll copies
@@ -609,7 +611,7 @@ __global__ void __launch_bounds__(TILE, 2)
         }
         if (threadIdx.x == 0) extra += sizeof(S) == 8 ? 4u : 3u;
         fresh = true;
-        if constexpr (!GANG) {  // apart from the update's, which so stays a straight line (FP64, 9,261 nodes: 4% of a step)
+        if constexpr (!GANG) {  // apart from the update's, which so stays a straight line (4% of an FP64 step, 9,261 nodes)
           if (!advance()) return;
           continue;
         }
